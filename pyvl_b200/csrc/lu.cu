@@ -21,10 +21,9 @@
 // speculative path on every panel; a bordered closed-body system falls back on the panel
 // holding the zero-diagonal border.
 //
-// The solve runs two wavefront kernels (forward with unit-lower L, backward with U) over
-// row blocks, one CTA per block, co-resident through a cooperative launch; each CTA stages
-// its diagonal block in shared memory before waiting, and every wait on an earlier block is
-// bounded and reports a time-out through a device error word.
+// The solve runs two wavefront kernels (trsv.cuh; forward with unit-lower L, backward with U) over
+// row blocks, one CTA per block, co-resident through a cooperative launch; every wait on an
+// earlier block is bounded and reports a time-out through a device error word.
 #include <algorithm>
 #include <cstdint>
 
@@ -49,8 +48,7 @@ struct LuWs {
     double* top_out;        // (NB, NB) speculative top block
     int32_t* reject;        // per panel: the speculation failed
     int32_t* ok;            // per panel: speculative factors accepted
-    int32_t* flags;         // wavefront flags (solve)
-    double* tmp;            // (n) solve vector
+    double* tmp;            // (n) vector of the blocked solve
     double* inv;            // (n_blocks, 2, kRB, kRB): inverses of the diagonal blocks of L and U
     double* backup_row;     // (NB, n) copy of the panel's row block right of it (FP64 path)
     double* linv;           // (NB, NB) inverse of the panel's unit-lower L11 (FP64 path)
@@ -61,7 +59,7 @@ size_t lu_ws_bytes(uint32_t n)
 {
     return align256((size_t)n * NB * sizeof(double)) + align256((size_t)NB * NB * sizeof(double)) +
            align256(((size_t)n / NB + 2) * sizeof(int32_t)) +
-           align256(((size_t)n / NB + 2) * sizeof(int32_t)) + align256(((size_t)n / kRB + 2) * sizeof(int32_t)) +
+           align256(((size_t)n / NB + 2) * sizeof(int32_t)) +
            align256((size_t)n * sizeof(double)) + align256(((size_t)n + kRB - 1) / kRB * 2 * kRB * kRB * sizeof(double)) +
            align256((size_t)NB * n * sizeof(double)) + 2 * align256((size_t)NB * NB * sizeof(double));
 }
@@ -78,8 +76,6 @@ LuWs carve(void* ws, uint32_t n)
     p += align256(((size_t)n / NB + 2) * sizeof(int32_t));
     w.ok = reinterpret_cast<int32_t*>(p);
     p += align256(((size_t)n / NB + 2) * sizeof(int32_t));
-    w.flags = reinterpret_cast<int32_t*>(p);
-    p += align256(((size_t)n / kRB + 2) * sizeof(int32_t));
     w.tmp = reinterpret_cast<double*>(p);
     p += align256((size_t)n * sizeof(double));
     w.inv = reinterpret_cast<double*>(p);
@@ -737,14 +733,14 @@ __global__ void __launch_bounds__(256) block_update_kernel(uint32_t n, uint32_t 
         x[r] -= s;
 }
 
-int coresident_blocks(const void* fn, int threads)
+int coresident_blocks(const void* fn, int threads, size_t smem)
 {
     int dev = 0, sms = 0, per = 0;
     if (cudaGetDevice(&dev) != cudaSuccess)
         return 0;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
         return 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, threads, 0) != cudaSuccess)
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, threads, smem) != cudaSuccess)
         return 0;
     return sms * per;
 }
@@ -879,27 +875,33 @@ extern "C" int pvl_lu_solve(uint32_t n, const double* LU, uint32_t lda, const in
     const uint32_t nblk = (n + kRB - 1) / kRB;
     const void* fwd = (const void*)pvl::trsv::wavefront_kernel<true>;
     const void* bwd = (const void*)pvl::trsv::wavefront_kernel<false>;
-    if ((int)nblk > coresident_blocks(fwd, kSolveThreads) || (int)nblk > coresident_blocks(bwd, kSolveThreads))
+    const size_t smem = pvl::trsv::kSmem;
+    PVL_SMEM_OPTIN(fwd, smem);
+    PVL_SMEM_OPTIN(bwd, smem);
+    if ((int)nblk > coresident_blocks(fwd, kSolveThreads, smem) || (int)nblk > coresident_blocks(bwd, kSolveThreads, smem))
         return pvl_fail(PVL_ERR_ARG, "pvl_lu_solve: n = %u needs %u co-resident blocks", n, nblk);
     cudaStream_t st = (cudaStream_t)stream;
     LuWs w = carve(ws, n);
-    const int32_t* perm = ipiv + n;
+    // y = L^-1 P b, then x = U^-1 y (also into b); both start as "not ready" (trsv.cuh)
+    double* y = w.backup;  // n x 64 doubles, free during the solve
+    double* x = y + n;
     PVL_CUDA_CHECK(cudaMemsetAsync(err, 0, sizeof(int32_t), st));
-    gather_kernel<<<blocks_for(n, 256), 256, 0, st>>>(n, perm, b, w.tmp);
-    PVL_LAUNCH_CHECK();
+    PVL_CUDA_CHECK(cudaMemsetAsync(y, pvl::trsv::kNotReadyByte, 2 * sizeof(double) * (size_t)n, st));
+    const double* iv = w.inv;
+    const int32_t* perm = ipiv + n;
+    const int32_t* no_perm = nullptr;
+    double* no_out = nullptr;
+    int32_t* no_flags = nullptr;
     long long spin = pvl::trsv::kSpinLimit;
     int32_t skip = -1;
-    for (int pass = 0; pass < 2; ++pass) {
-        PVL_CUDA_CHECK(cudaMemsetAsync(w.flags, 0, sizeof(int32_t) * (nblk + 1), st));
-        double* xt = w.tmp;
-        int32_t* fl = w.flags;
-        const double* iv = w.inv;
-        void* args[] = {(void*)&n, (void*)&LU, (void*)&lda, (void*)&iv, (void*)&xt, (void*)&fl, (void*)&err,
-                        (void*)&spin, (void*)&skip};
-        PVL_CUDA_CHECK(cudaLaunchCooperativeKernel(pass == 0 ? fwd : bwd, dim3(nblk), dim3(kSolveThreads), args, 0, st));
-        pvl_count_launch();
-    }
-    PVL_CUDA_CHECK(cudaMemcpyAsync(b, w.tmp, sizeof(double) * n, cudaMemcpyDeviceToDevice, st));
+    void* fargs[] = {(void*)&n, (void*)&LU, (void*)&lda, (void*)&iv, (void*)&b, (void*)&perm, (void*)&y,
+                     (void*)&no_out, (void*)&no_flags, (void*)&err, (void*)&spin, (void*)&skip};
+    PVL_CUDA_CHECK(cudaLaunchCooperativeKernel(fwd, dim3(nblk), dim3(kSolveThreads), fargs, smem, st));
+    pvl_count_launch();
+    void* bargs[] = {(void*)&n, (void*)&LU, (void*)&lda, (void*)&iv, (void*)&y, (void*)&no_perm, (void*)&x,
+                     (void*)&b, (void*)&no_flags, (void*)&err, (void*)&spin, (void*)&skip};
+    PVL_CUDA_CHECK(cudaLaunchCooperativeKernel(bwd, dim3(nblk), dim3(kSolveThreads), bargs, smem, st));
+    pvl_count_launch();
     return PVL_OK;
 }
 

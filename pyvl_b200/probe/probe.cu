@@ -5,7 +5,7 @@
 // are measured against.  pvl_probe_far_series() runs the FP64 reciprocal and arctangent series
 // of the pair kernels (pvl::FarSeries) on given arguments, so that a test can hold them to
 // their error bounds.  pvl_probe_trsv_timeout() launches the product's wavefront triangular
-// solve (trsv.cuh) with a short spin limit and one row block that never publishes its flag,
+// solve (trsv.cuh) with a short spin limit and one row block that never stores its solution,
 // so that a test can watch every later block's bounded wait run out and report through the
 // error word, with no GPU fault and nothing left running.  pvl_probe_gemm_timeout() runs the
 // product's TMA-fed TF32 GEMM (gemm_tc.cuh, through its launcher in libpvl_b200.so) with a
@@ -65,6 +65,10 @@ __global__ void far_series_kernel(uint32_t n, const double* __restrict__ x, cons
         sum[i] = pvl::FarSeries<double>::sum(w[i]);
     }
 }
+
+// The wavefront solve's "not ready" solution vector (the product keeps it in the LU workspace).
+constexpr uint32_t kTrsvMax = 16384;
+__device__ double g_trsv_x[kTrsvMax];
 }  // namespace
 
 extern "C" const char* pvl_probe_last_error(void) { return g_err; }
@@ -104,14 +108,15 @@ extern "C" int pvl_probe_trsv_timeout(uint32_t n, const double* LU, uint32_t lda
                                       int32_t* flags, int32_t* err, long long spin_limit, int32_t skip_block,
                                       int lower, void* stream)
 {
-    if (n == 0 || !LU || !inv || !x || !flags || !err || lda < n || spin_limit <= 0)
+    if (n == 0 || !LU || !inv || !x || !flags || !err || lda < n || spin_limit <= 0 || n > kTrsvMax)
         return fail(PVL_ERR_ARG, "pvl_probe_trsv_timeout: bad arguments");
     const uint32_t nblk = (n + pvl::trsv::kRB - 1) / pvl::trsv::kRB;
     const void* fn = lower ? (const void*)pvl::trsv::wavefront_kernel<true> : (const void*)pvl::trsv::wavefront_kernel<false>;
     int dev = 0, sms = 0, per = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, pvl::trsv::kThreads, 0) != cudaSuccess)
+        cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pvl::trsv::kSmem) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, pvl::trsv::kThreads, pvl::trsv::kSmem) != cudaSuccess)
         return fail(PVL_ERR_CUDA, "pvl_probe_trsv_timeout: occupancy query failed");
     if ((long long)nblk > (long long)sms * per)
         return fail(PVL_ERR_ARG, "pvl_probe_trsv_timeout: %u blocks cannot be co-resident", nblk);
@@ -119,9 +124,14 @@ extern "C" int pvl_probe_trsv_timeout(uint32_t n, const double* LU, uint32_t lda
     if (cudaMemsetAsync(flags, 0, sizeof(int32_t) * (nblk + 1), st) != cudaSuccess ||
         cudaMemsetAsync(err, 0, sizeof(int32_t), st) != cudaSuccess)
         return fail(PVL_ERR_CUDA, "pvl_probe_trsv_timeout: memset failed");
-    void* args[] = {(void*)&n, (void*)&LU, (void*)&lda, (void*)&inv, (void*)&x, (void*)&flags, (void*)&err,
-                    (void*)&spin_limit, (void*)&skip_block};
-    if (cudaLaunchCooperativeKernel(fn, dim3(nblk), dim3(pvl::trsv::kThreads), args, 0, st) != cudaSuccess)
+    double* sol = nullptr;
+    if (cudaGetSymbolAddress((void**)&sol, g_trsv_x) != cudaSuccess ||
+        cudaMemsetAsync(sol, pvl::trsv::kNotReadyByte, sizeof(double) * n, st) != cudaSuccess)
+        return fail(PVL_ERR_CUDA, "pvl_probe_trsv_timeout: solution buffer");
+    const int32_t* perm = nullptr;
+    void* args[] = {(void*)&n, (void*)&LU, (void*)&lda, (void*)&inv, (void*)&x, (void*)&perm, (void*)&sol, (void*)&x,
+                    (void*)&flags, (void*)&err, (void*)&spin_limit, (void*)&skip_block};
+    if (cudaLaunchCooperativeKernel(fn, dim3(nblk), dim3(pvl::trsv::kThreads), args, pvl::trsv::kSmem, st) != cudaSuccess)
         return fail(PVL_ERR_CUDA, "pvl_probe_trsv_timeout: launch failed");
     return PVL_OK;
 }
