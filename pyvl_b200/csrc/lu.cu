@@ -2,24 +2,19 @@
 // system matrix the induction kernels write.  Replaces the reference's
 // scipy.linalg.lu_factor / lu_solve (python/pyvl/solver.py:223-227).
 //
-// Right-looking blocked factorisation, panel width NB = 64.  Per panel (k0, nb):
-//   1. panel_spec_kernel -- speculative factorisation of the whole panel with the diagonal as
-//      pivot.  Every CTA factors the same nb x nb top block (one row per thread, rows held in
-//      registers) together with its own 64 rows below it, so no CTA waits for another.  Per
-//      column it records the largest |entry| below the diagonal at the moment the column is
-//      eliminated.
-//   2. panel_pivot_kernel -- one CTA: if every diagonal entry is non-zero and no entry below
-//      it is larger, partial pivoting would have chosen exactly these pivots (LAPACK's idamax
-//      returns the first maximal entry and the diagonal comes first), so the speculative
-//      factors ARE the GEPP factors: commit them with identity pivots.  Otherwise restore the
-//      panel from the backup and factor it with explicit partial pivoting in getf2 order.
-//   3. trsm_kernel -- applies the panel's interchanges to the other columns and forms
-//      U12 = L11^-1 A12 (one column per thread, held in registers).
-//   4. gemm_update_kernel -- A22 -= L21 U12, FP64, 128 x 128 tiles, 8 x 8 outputs per thread,
-//      128-bit conflict-free shared loads.
-// Diagonally dominant systems (the vortex-ring matrices are close to -2 pi I) take the
-// speculative path on every panel; a bordered closed-body system falls back on the panel
-// holding the zero-diagonal border.
+// Right-looking blocked factorisation, panel width NB = 64, one panel of look-ahead.  Per panel:
+//   1. the diagonal block and its inverses, and 2. the multipliers and the row block, as if no
+//      row interchange were needed (lu_panel.cuh), each fused with the previous panel's update;
+//   3. panel_pivot_kernel -- if partial pivoting would have chosen other rows (some multiplier
+//      not below 1 in magnitude), the panel is restored from its backup and factored with
+//      explicit partial pivoting in getf2 order;
+//   4. trsm_kernel -- that panel's interchanges applied to the other columns and its
+//      U12 = L11^-1 A12 by substitution (nothing to do for an accepted panel);
+//   5. dmma_update_kernel -- A22 -= L21 U12 beyond the next panel, on a side stream beside the
+//      next panel's steps 1 and 2.
+// Diagonally dominant systems (the vortex-ring matrices are close to -2 pi I) are accepted on
+// every panel; a bordered closed-body system falls back on the panel holding the zero-diagonal
+// border.  The FP32 factorisation below keeps its own panel kernel (panel_spec_kernel).
 //
 // The solve runs two wavefront kernels (trsv.cuh; forward with unit-lower L, backward with U) over
 // row blocks, one CTA per block, co-resident through a cooperative launch; every wait on an
@@ -29,6 +24,7 @@
 
 #include "pvl_common.cuh"
 #include "dmma.cuh"
+#include "lu_panel.cuh"
 #include "trsv.cuh"
 
 namespace {
@@ -37,7 +33,7 @@ constexpr int NB = 64;               // panel width
 constexpr int kSlabRows = 64;        // rows below the top block per CTA in panel_spec_kernel
 constexpr int kRB = 64;              // rows per block in the wavefront solves
 static_assert(kRB == pvl::trsv::kRB, "the solve's row blocks are the inverted diagonal blocks");
-static_assert(NB == pvl::dmma::K, "the tensor-core products have K = the panel width");
+static_assert(NB == pvl::dmma::K && NB == pvl::panel::NB, "the tensor-core products have K = the panel width");
 constexpr int kSolveThreads = pvl::trsv::kThreads;
 
 inline size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
@@ -45,15 +41,17 @@ inline unsigned blocks_for(size_t n, unsigned t) { return (unsigned)((n + t - 1)
 
 struct LuWs {
     double* backup;         // (n, NB) copy of the current panel before speculation
-    double* top_out;        // (NB, NB) speculative top block
+    double* top_out;        // (NB, NB) speculative top block (FP32 path)
     int32_t* reject;        // per panel: the speculation failed
     int32_t* ok;            // per panel: speculative factors accepted
     double* tmp;            // (n) vector of the blocked solve
     double* inv;            // (n_blocks, 2, kRB, kRB): inverses of the diagonal blocks of L and U
     double* backup_row;     // (NB, n) copy of the panel's row block right of it (FP64 path)
-    double* linv;           // (NB, NB) inverse of the panel's unit-lower L11 (FP64 path)
-    double* uinv;           // (NB, NB) inverse of the panel's U11 (FP64 path)
+    double* even;           // (n, even_stride(n)) for odd n: the matrix with 128-byte rows (FP64 path)
 };
+
+// Row stride of LuWs::even, 0 where the matrix is factored in place.
+uint32_t even_stride(uint32_t n) { return n % 2 ? (n + 15) & ~15u : 0; }
 
 size_t lu_ws_bytes(uint32_t n)
 {
@@ -61,7 +59,7 @@ size_t lu_ws_bytes(uint32_t n)
            align256(((size_t)n / NB + 2) * sizeof(int32_t)) +
            align256(((size_t)n / NB + 2) * sizeof(int32_t)) +
            align256((size_t)n * sizeof(double)) + align256(((size_t)n + kRB - 1) / kRB * 2 * kRB * kRB * sizeof(double)) +
-           align256((size_t)NB * n * sizeof(double)) + 2 * align256((size_t)NB * NB * sizeof(double));
+           align256((size_t)NB * n * sizeof(double)) + align256((size_t)n * even_stride(n) * sizeof(double));
 }
 
 LuWs carve(void* ws, uint32_t n)
@@ -82,9 +80,7 @@ LuWs carve(void* ws, uint32_t n)
     p += align256(((size_t)n + kRB - 1) / kRB * 2 * kRB * kRB * sizeof(double));
     w.backup_row = reinterpret_cast<double*>(p);
     p += align256((size_t)NB * n * sizeof(double));
-    w.linv = reinterpret_cast<double*>(p);
-    p += align256((size_t)NB * NB * sizeof(double));
-    w.uinv = reinterpret_cast<double*>(p);
+    w.even = reinterpret_cast<double*>(p);
     return w;
 }
 
@@ -93,6 +89,17 @@ __global__ void init_perm_kernel(uint32_t n, int32_t* __restrict__ perm)
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n)
         perm[i] = (int32_t)i;
+}
+
+// dst (row stride ldd) = src (row stride lds), n x n.
+__global__ void __launch_bounds__(256) copy_matrix_kernel(uint32_t n, const double* __restrict__ src, uint32_t lds,
+                                                          double* __restrict__ dst, uint32_t ldd)
+{
+    const uint32_t c = blockIdx.x * 256 + threadIdx.x;
+    if (c >= n)
+        return;
+    for (uint32_t r = blockIdx.y; r < n; r += gridDim.y)
+        dst[(size_t)r * ldd + c] = src[(size_t)r * lds + c];
 }
 
 // ---------------------------------------------------------------- 1+2. speculative panel
@@ -175,6 +182,12 @@ __global__ void __launch_bounds__(2 * kSlabRows) panel_spec_kernel(uint32_t n, u
 }
 
 // ---------------------------------------------------------------- 3. accept or pivot
+// top_out: the speculative top block, committed here if the panel is accepted (FP32 path); NULL:
+// the top block (and its identity pivots) is in A already, its old values in rows 0 .. 63 of backup.
+// A rejected panel of at most stage_rows rows is factored in shared memory (stage_rows x (NB + 1)
+// values of it): a column step is a chain of dependent passes over the panel, ~0.5 us each from
+// shared memory and several from L2 (the last full panel of a closed body's bordered system, 65
+// rows: 3.9 ms with one thread per row in global memory).
 template <typename T>
 __global__ void __launch_bounds__(1024) panel_pivot_kernel(uint32_t n, uint32_t k0, uint32_t nb, T* __restrict__ A,
                                                            uint32_t lda, const T* __restrict__ backup,
@@ -183,16 +196,20 @@ __global__ void __launch_bounds__(1024) panel_pivot_kernel(uint32_t n, uint32_t 
                                                            int32_t* __restrict__ ok, uint32_t panel,
                                                            int32_t* __restrict__ ipiv, int32_t* __restrict__ perm,
                                                            int32_t* __restrict__ info,
-                                                           const T* __restrict__ backup_row)
+                                                           const T* __restrict__ backup_row, uint32_t stage_rows)
 {
+    extern __shared__ __align__(16) unsigned char pivot_smem[];
     __shared__ T s_val[32];
     __shared__ uint32_t s_idx[32];
-    __shared__ uint32_t s_piv;
+    __shared__ uint32_t s_piv, s_pivs[NB], s_slot[NB];
+    __shared__ int32_t s_top[NB], s_ext[NB];
     __shared__ T s_prow[NB];
     const int bad = reject[panel];
     if (!bad) {
         if (threadIdx.x == 0)
             ok[panel] = 1;
+        if (!top_out)
+            return;
         for (uint32_t t = threadIdx.x; t < nb * nb; t += blockDim.x) {
             const uint32_t r = t / nb, c = t % nb;
             A[(size_t)(k0 + r) * lda + k0 + c] = top_out[(size_t)r * NB + c];
@@ -203,25 +220,32 @@ __global__ void __launch_bounds__(1024) panel_pivot_kernel(uint32_t n, uint32_t 
     }
     if (threadIdx.x == 0)
         ok[panel] = 0;
-    // the top block of A was never written; restore the rows below it, then LAPACK getf2:
-    // first row of maximal |a|, swap, scale, update
-    for (size_t t = threadIdx.x; t < (size_t)(n - k0 - nb) * nb; t += blockDim.x) {
-        const uint32_t r = (uint32_t)(t / nb) + nb, c = (uint32_t)(t % nb);
-        A[(size_t)(k0 + r) * lda + k0 + c] = backup[(size_t)r * NB + c];
+    // restore what was overwritten (with top_out, the top block of A was not), in place or in shared
+    // memory, then LAPACK getf2: first row of maximal |a|, swap, scale, update
+    const uint32_t rows = n - k0;
+    const bool staged = rows <= stage_rows;
+    T* M = staged ? reinterpret_cast<T*>(pivot_smem) : A + (size_t)k0 * lda + k0;
+    const size_t ldm = staged ? NB + 1 : lda;
+    const uint32_t r_first = top_out ? nb : 0;
+    for (size_t t = threadIdx.x; t < (size_t)rows * nb; t += blockDim.x) {
+        const uint32_t r = (uint32_t)(t / nb), c = (uint32_t)(t % nb);
+        if (r >= r_first)
+            M[r * ldm + c] = backup[(size_t)r * NB + c];
+        else if (staged)
+            M[r * ldm + c] = A[(size_t)(k0 + r) * lda + k0 + c];
     }
     if (backup_row)  // the FP64 path also replaced the row block right of the panel by U12
-        for (size_t t = threadIdx.x; t < (size_t)nb * (n - k0 - nb); t += blockDim.x) {
-            const uint32_t r = (uint32_t)(t / (n - k0 - nb)), c = k0 + nb + (uint32_t)(t % (n - k0 - nb));
+        for (size_t t = threadIdx.x; t < (size_t)nb * (rows - nb); t += blockDim.x) {
+            const uint32_t r = (uint32_t)(t / (rows - nb)), c = k0 + nb + (uint32_t)(t % (rows - nb));
             A[(size_t)(k0 + r) * lda + c] = backup_row[(size_t)r * n + c];
         }
     __syncthreads();
-    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n_warps = blockDim.x >> 5;
     for (uint32_t j = 0; j < nb; ++j) {
-        const uint32_t col = k0 + j;
         T best = T(-1);
         uint32_t bidx = 0xFFFFFFFFu;
-        for (uint32_t r = col + threadIdx.x; r < n; r += blockDim.x) {
-            const T v = fabs(A[(size_t)r * lda + col]);
+        for (uint32_t r = j + threadIdx.x; r < rows; r += blockDim.x) {
+            const T v = fabs(M[r * ldm + j]);
             if (v > best) {
                 best = v;
                 bidx = r;
@@ -240,51 +264,112 @@ __global__ void __launch_bounds__(1024) panel_pivot_kernel(uint32_t n, uint32_t 
             s_idx[warp] = bidx;
         }
         __syncthreads();
-        if (threadIdx.x == 0) {
-            T b = T(-1);
-            uint32_t bi = col;
-            for (uint32_t w = 0; w < blockDim.x / 32; ++w)
-                if (s_val[w] > b || (s_val[w] == b && s_idx[w] < bi)) {
-                    b = s_val[w];
-                    bi = s_idx[w];
+        if (warp == 0) {
+            T b = lane < n_warps ? s_val[lane] : T(-1);
+            uint32_t bi = lane < n_warps ? s_idx[lane] : 0xFFFFFFFFu;
+            for (int o = 16; o > 0; o >>= 1) {
+                const T ov = __shfl_xor_sync(0xffffffffu, b, o);
+                const uint32_t oi = __shfl_xor_sync(0xffffffffu, bi, o);
+                if (ov > b || (ov == b && oi < bi)) {
+                    b = ov;
+                    bi = oi;
                 }
-            s_piv = bi;
-            ipiv[col] = (int32_t)bi;
-            if (bi != col) {
-                const int32_t t = perm[col];
-                perm[col] = perm[bi];
-                perm[bi] = t;
+            }
+            if (lane == 0) {
+                bi = bi < rows ? bi : j;  // nothing compared greater (NaNs): no interchange
+                s_piv = s_pivs[j] = bi;
+                ipiv[k0 + j] = (int32_t)(k0 + bi);
             }
         }
         __syncthreads();
         const uint32_t p = s_piv;
-        if (p != col)
-            for (uint32_t c = threadIdx.x; c < nb; c += blockDim.x) {
-                const T a = A[(size_t)col * lda + k0 + c];
-                A[(size_t)col * lda + k0 + c] = A[(size_t)p * lda + k0 + c];
-                A[(size_t)p * lda + k0 + c] = a;
+        for (uint32_t c = threadIdx.x; c < nb; c += blockDim.x) {
+            const T a = M[p * ldm + c];
+            s_prow[c] = a;
+            if (p != j) {
+                M[p * ldm + c] = M[j * ldm + c];
+                M[j * ldm + c] = a;
             }
-        __syncthreads();
-        for (uint32_t c = threadIdx.x; c < nb; c += blockDim.x)
-            s_prow[c] = A[(size_t)col * lda + k0 + c];
+        }
         __syncthreads();
         const T piv = s_prow[j];
         if (piv == T(0)) {
             if (threadIdx.x == 0)
-                atomicCAS(info, 0, (int32_t)(col + 1));
+                atomicCAS(info, 0, (int32_t)(k0 + j + 1));
             __syncthreads();
             continue;
         }
         const T rcp = T(1) / piv;
-        for (uint32_t r = col + 1 + threadIdx.x; r < n; r += blockDim.x) {
-            T* row = A + (size_t)r * lda + k0;
-            const T l = row[j] * rcp;
-            row[j] = l;
-            for (uint32_t c = j + 1; c < nb; ++c)
-                row[c] -= l * s_prow[c];
+        for (uint32_t r = j + 1 + threadIdx.x; r < rows; r += blockDim.x)
+            M[r * ldm + j] *= rcp;
+        __syncthreads();
+        // a warp per row, two columns per lane, kRowsAhead rows in flight
+        constexpr uint32_t kRowsAhead = 4;
+        const uint32_t c0 = j + 1 + lane, c1 = c0 + 32;
+        const T p0 = c0 < nb ? s_prow[c0] : T(0), p1 = c1 < nb ? s_prow[c1] : T(0);
+        for (uint32_t r = j + 1 + warp; r < rows; r += kRowsAhead * n_warps) {
+            T l[kRowsAhead], a[kRowsAhead][2];
+#pragma unroll
+            for (uint32_t u = 0; u < kRowsAhead; ++u) {
+                const uint32_t rr = r + u * n_warps;
+                const bool in = rr < rows;
+                l[u] = in ? M[rr * ldm + j] : T(0);
+                a[u][0] = in && c0 < nb ? M[rr * ldm + c0] : T(0);
+                a[u][1] = in && c1 < nb ? M[rr * ldm + c1] : T(0);
+            }
+#pragma unroll
+            for (uint32_t u = 0; u < kRowsAhead; ++u) {
+                const uint32_t rr = r + u * n_warps;
+                if (rr < rows && c0 < nb)
+                    M[rr * ldm + c0] = a[u][0] - l[u] * p0;
+                if (rr < rows && c1 < nb)
+                    M[rr * ldm + c1] = a[u][1] - l[u] * p1;
+            }
         }
         __syncthreads();
     }
+    if (staged)
+        for (uint32_t t = threadIdx.x; t < rows * nb; t += blockDim.x) {
+            const uint32_t r = t / nb, c = t % nb;
+            A[(size_t)(k0 + r) * lda + k0 + c] = M[r * ldm + c];
+        }
+    // the panel's interchanges in perm: they touch its first nb entries (s_top) and those of the pivot
+    // rows below (s_ext, one slot per distinct row: the first j that chose it)
+    const uint32_t j = threadIdx.x;
+    if (j < nb) {
+        const uint32_t bi = s_pivs[j];
+        uint32_t slot = j;
+        for (uint32_t i = nb; i-- > 0;)
+            if (s_pivs[i] == bi)
+                slot = i;
+        s_slot[j] = slot;
+        s_top[j] = perm[k0 + j];
+        s_ext[j] = perm[k0 + bi];
+    }
+    __syncthreads();
+    if (threadIdx.x == 0)
+        for (uint32_t i = 0; i < nb; ++i) {
+            const uint32_t bi = s_pivs[i];
+            int32_t& other = bi < nb ? s_top[bi] : s_ext[s_slot[i]];
+            const int32_t t = s_top[i];
+            s_top[i] = other;
+            other = t;
+        }
+    __syncthreads();
+    if (j < nb) {
+        perm[k0 + j] = s_top[j];
+        if (s_pivs[j] >= nb && s_slot[j] == j)
+            perm[k0 + s_pivs[j]] = s_ext[j];
+    }
+}
+
+// Rows that a rejected panel may have to be factored in shared memory.
+constexpr uint32_t kPivotStageRows = 432;
+
+template <typename T>
+size_t pivot_smem(uint32_t rows)
+{
+    return rows <= kPivotStageRows ? (size_t)rows * (NB + 1) * sizeof(T) : 0;
 }
 
 // ---------------------------------------------------------------- 3. swaps + U12
@@ -359,206 +444,13 @@ __global__ void __launch_bounds__(kTrsmCols, 1) trsm_kernel(uint32_t n, uint32_t
     }
 }
 
-// ---------------------------------------------------------------- FP64 panel on the tensor cores
+// ---------------------------------------------------------------- FP64 panels and updates
 // The FP64 factorisation first factors each panel without interchanges and then checks that
 // partial pivoting would have made none: with no interchange before column j, GEPP keeps the
 // diagonal in column j exactly when no entry below it is larger in magnitude at that moment,
 // i.e. when every multiplier l_ij (i > j) has |l_ij| <= 1 (LAPACK's idamax returns the first
-// maximal entry, and the diagonal comes first).  The multipliers are formed by blocks:
-//   top_factor_kernel   L11 U11 = A11 (one CTA, the 64 x 64 diagonal block, in registers),
-//                       the check inside the block, and L11^-1, U11^-1;
-//   panel_apply_kernel  L21 = A21 U11^-1 (with the check on every multiplier) and
-//                       U12 = L11^-1 A12, both as FP64 tensor-core tiles (dmma.cuh), the
-//                       overwritten operands backed up;
-//   panel_pivot_kernel  commits the top block -- or, if any check failed, restores the panel and
-//                       its row block and refactors the panel with explicit partial pivoting in
-//                       getf2 order, after which trsm_kernel applies the interchanges and forms
-//                       U12 by substitution;
-//   dmma_update_kernel  A22 -= L21 U12 on the FP64 tensor cores: 64 x 64 tiles, each CTA a
-//                       run of them with the next tile's operands loading during the MMAs.
-// Every product has K = 64, the panel width; the multipliers and U12 are the blocked forms of
-// getf2's and trsm's, equal to them up to rounding.
-// Columns per thread of the top-block kernel: 16 (256 threads), 8 (512) or 4 (1024); more
-// threads shorten each column step's chain of dependent instructions per warp.
-#ifndef PVL_TOP_CPT
-#define PVL_TOP_CPT 16
-#endif
-constexpr int kTopCpt = PVL_TOP_CPT;
-constexpr int kTopGroups = NB / kTopCpt;          // threads per row (neighbouring lanes)
-constexpr int kTopThreads = NB * kTopGroups;
-constexpr int kTopGs = kTopCpt + 2;               // doubles per column group of a broadcast row:
-                                                  // the groups' 16-byte loads fall in distinct banks
-static_assert(kTopCpt == 16 || kTopCpt == 8 || kTopCpt == 4, "16, 8 or 4 columns per thread");
-
-constexpr double kPivotLo = 0x1p-1000, kPivotHi = 0x1p+1000;
-
-// 1/p for a pivot with kPivotLo <= |p| <= kPivotHi: the hardware's approximate reciprocal r
-// (rcp.approx.ftz.f64, relative error d < 2^-19) refined by one third-order step of the
-// geometric series 1/p = r / (1 - e), e = 1 - p r:  r + r (e + e^2) = (1/p)(1 - d^3), within an
-// ulp of the rounded quotient.  Pivots outside the range take the exact (pivoting) path.
-__device__ __forceinline__ double pivot_rcp(double p)
-{
-    double r;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(p));
-    const double e = fma(-p, r, 1.0);
-    return fma(r, fma(e, e, e), r);
-}
-
-// One CTA: the 64 x 64 diagonal block (a partial block padded with identity) factored without
-// interchanges, with X = L11^-1 and Y = U11^-1 formed in the same 64 column steps.  Thread
-// (r, g) holds row r, columns C g .. C g + C - 1 (C = kTopCpt), of T, X and Y in registers (the
-// threads of a row are neighbouring lanes); the column loop is unrolled by C, so every register
-// index is a constant.  Step j: row j is final and sits in shared memory (published by its
-// threads at the end of step j - 1, double-buffered by parity, one barrier per step).  A row
-// r > j takes its multiplier l = T[r][j] / U[j][j] (by the pivot's reciprocal, as getf2) from
-// the thread that holds column j, checks it, and applies T[r][c] -= l U[j][c] (c > j) and
-// X[r] -= l X[j].  A row r <= j finishes Y[r][j] = (delta_rj - sum_{k<j} Y[r][k] U[k][j]) /
-// U[j][j] (the sum has been accumulated in y by the earlier steps) and applies
-// Y[r][c] -= Y[r][j] U[j][c] (c > j), the same broadcast row.  The threads of row j + 1 then
-// publish it with its pivot's reciprocal.
-__global__ void __launch_bounds__(kTopThreads) top_factor_kernel(uint32_t k0, uint32_t nb,
-                                                                 const double* __restrict__ A, uint32_t lda,
-                                                                 double* __restrict__ top_out,
-                                                                 double* __restrict__ linv,
-                                                                 double* __restrict__ uinv,
-                                                                 int32_t* __restrict__ reject)
-{
-    constexpr int C = kTopCpt, G = kTopGroups;
-    __shared__ __align__(16) double prow[2][G][kTopGs];  // row j of T
-    __shared__ __align__(16) double xrow[2][G][kTopGs];  // row j of X
-    __shared__ double rd[NB];                            // 1 / U[q][q]
-    const uint32_t tid = threadIdx.x, row = tid / G, g = tid % G;
-    const int src = (int)(tid & 31u & ~(uint32_t)(G - 1));  // lane of this row's group 0
-    double t[C], x[C], y[C];
-#pragma unroll
-    for (int k = 0; k < C; ++k) {
-        const uint32_t c = C * g + k;
-        t[k] = (row < nb && c < nb) ? A[(size_t)(k0 + row) * lda + k0 + c] : (row == c ? 1.0 : 0.0);
-        x[k] = y[k] = row == c ? 1.0 : 0.0;
-    }
-    bool bad = false;
-    if (row == 0) {
-#pragma unroll
-        for (int k = 0; k < C; k += 2) {
-            *reinterpret_cast<double2*>(&prow[0][g][k]) = make_double2(t[k], t[k + 1]);
-            *reinterpret_cast<double2*>(&xrow[0][g][k]) = make_double2(x[k], x[k + 1]);
-        }
-        if (g == 0) {
-            bad |= !(fabs(t[0]) >= kPivotLo && fabs(t[0]) <= kPivotHi);  // zero, tiny, huge or NaN pivot
-            rd[0] = pivot_rcp(t[0]);
-        }
-    }
-    __syncthreads();
-#pragma unroll 1
-    for (uint32_t gj = 0; gj < (uint32_t)G; ++gj) {
-#pragma unroll
-        for (int kj = 0; kj < C; ++kj) {
-            const uint32_t j = C * gj + kj;
-            const int b = kj & 1;
-            const bool below = row > j;
-            const double a = __shfl_sync(0xffffffffu, below ? t[kj] : y[kj], src + (int)gj) * rd[j];
-            if (g == gj) {
-                if (below) {
-                    bad |= !(fabs(a) < pvl::dmma::kMultLimit);
-                    t[kj] = a;
-                } else {
-                    y[kj] = a;
-                }
-            }
-            if (g >= gj) {  // columns right of j: k > kj in group gj, every k in later groups
-                const bool later = g > gj;
-                if (below) {
-#pragma unroll
-                    for (int k = 0; k < C; k += 2) {
-                        const double2 p = *reinterpret_cast<const double2*>(&prow[b][g][k]);
-                        if (k > kj || later)
-                            t[k] = fma(-a, p.x, t[k]);
-                        if (k + 1 > kj || later)
-                            t[k + 1] = fma(-a, p.y, t[k + 1]);
-                    }
-                } else {
-#pragma unroll
-                    for (int k = 0; k < C; k += 2) {
-                        const double2 p = *reinterpret_cast<const double2*>(&prow[b][g][k]);
-                        if (k > kj || later)
-                            y[k] = fma(-a, p.x, y[k]);
-                        if (k + 1 > kj || later)
-                            y[k + 1] = fma(-a, p.y, y[k + 1]);
-                    }
-                }
-            }
-            if (below && g <= gj) {  // X[j][c] = 0 for c > j
-#pragma unroll
-                for (int k = 0; k < C; k += 2) {
-                    const double2 p = *reinterpret_cast<const double2*>(&xrow[b][g][k]);
-                    x[k] = fma(-a, p.x, x[k]);
-                    x[k + 1] = fma(-a, p.y, x[k + 1]);
-                }
-            }
-            if (row == j + 1) {  // row j + 1 is final: publish it (never true after the last step)
-                const int kn = (kj + 1) % C;
-                const uint32_t gn = gj + (kj == C - 1 ? 1u : 0u);
-#pragma unroll
-                for (int k = 0; k < C; k += 2) {
-                    *reinterpret_cast<double2*>(&prow[b ^ 1][g][k]) = make_double2(t[k], t[k + 1]);
-                    *reinterpret_cast<double2*>(&xrow[b ^ 1][g][k]) = make_double2(x[k], x[k + 1]);
-                }
-                if (g == gn) {
-                    bad |= !(fabs(t[kn]) >= kPivotLo && fabs(t[kn]) <= kPivotHi);
-                    rd[j + 1] = pivot_rcp(t[kn]);
-                }
-            }
-            __syncthreads();
-        }
-    }
-    if (__syncthreads_or(bad) && tid == 0)
-        atomicExch(reject, 1);
-    const size_t o = (size_t)row * NB + C * g;
-#pragma unroll
-    for (int k = 0; k < C; k += 2) {
-        *reinterpret_cast<double2*>(linv + o + k) = make_double2(x[k], x[k + 1]);
-        *reinterpret_cast<double2*>(uinv + o + k) = make_double2(y[k], y[k + 1]);
-    }
-    if (row < nb) {
-#pragma unroll
-        for (int k = 0; k < C; ++k)
-            if (C * g + k < nb)
-                top_out[o + k] = t[k];
-    }
-}
-
-constexpr int kApplyRows = 32;  // L21 tile: 32 rows x 64
-constexpr int kApplyCols = 32;  // U12 tile: 64 x 32 columns
-constexpr size_t kApplySmem = sizeof(pvl::dmma::Smem<64, 32>) > sizeof(pvl::dmma::Smem<32, 64>)
-                                  ? sizeof(pvl::dmma::Smem<64, 32>) : sizeof(pvl::dmma::Smem<32, 64>);
-
-// CTAs 0 .. n_ltiles-1: a 32-row tile of L21 = A21 U11^-1; the rest: a 32-column tile of
-// U12 = L11^-1 A12.  Both in place, the old values backed up for the pivoting fallback.
-template <bool VEC>
-__global__ void __launch_bounds__(pvl::dmma::kThreads) panel_apply_kernel(uint32_t n, uint32_t k0,
-                                                                          double* __restrict__ A, uint32_t lda,
-                                                                          const double* __restrict__ linv,
-                                                                          const double* __restrict__ uinv,
-                                                                          double* __restrict__ backup,
-                                                                          double* __restrict__ backup_row,
-                                                                          int32_t* __restrict__ reject,
-                                                                          uint32_t n_ltiles)
-{
-    using namespace pvl::dmma;
-    extern __shared__ __align__(16) double apply_smem[];
-    const uint32_t base = k0 + NB;
-    if (blockIdx.x < n_ltiles) {
-        auto& sm = *reinterpret_cast<Smem<kApplyRows, 64>*>(apply_smem);
-        const uint32_t r0 = base + blockIdx.x * kApplyRows;
-        tile<kApplyRows, 64, kLowerMul, VEC>(sm, A, lda, r0, k0, uinv, NB, 0, 0, A, lda, r0, k0,
-                                             min((uint32_t)kApplyRows, n - r0), NB, backup, k0, 0, 0, reject);
-    } else {
-        auto& sm = *reinterpret_cast<Smem<64, kApplyCols>*>(apply_smem);
-        const uint32_t c0 = base + (blockIdx.x - n_ltiles) * kApplyCols;
-        tile<64, kApplyCols, kUpperMul, VEC>(sm, linv, NB, 0, 0, A, lda, k0, c0, A, lda, k0, c0, NB,
-                                             min((uint32_t)kApplyCols, n - c0), backup_row, 0, 0, n, nullptr);
-    }
-}
+// maximal entry, and the diagonal comes first).  The multipliers and U12 are the blocked forms
+// of getf2's and trsm's (lu_panel.cuh), equal to them up to rounding.
 
 // One rectangle of the trailing update A22 -= L21 U12: C = rows row0 .. row0 + m, columns
 // col0 .. col0 + nn; A = the panel's L21 (columns a_col ..) on C's rows, B = its U12 (rows
@@ -577,30 +469,31 @@ UpdRect upd_rect(uint32_t row0, uint32_t col0, uint32_t m, uint32_t nn, uint32_t
 }
 
 // One CTA per SM, each a run of tiles (dmma.cuh update_tiles: C and A blocks stream into shared
-// memory one tile ahead of the MMAs).  CTA s < r0.slots runs tiles [s per, (s + 1) per) of r0,
-// the CTAs after them those of r1 (each rectangle's tiles in column-major order).
+// memory one tile ahead of the MMAs), in column-major order.
 template <bool VEC>
 __global__ void __launch_bounds__(pvl::dmma::kUpdThreads, 1) dmma_update_kernel(double* __restrict__ A, uint32_t lda,
-                                                                            UpdRect r0, UpdRect r1)
+                                                                            UpdRect r)
 {
     extern __shared__ __align__(16) double upd_smem[];
     auto& sm = *reinterpret_cast<pvl::dmma::UpdSmem*>(upd_smem);
-    uint32_t slot = blockIdx.x;
-    const bool first = slot < r0.slots;
-    const UpdRect r = first ? r0 : r1;
-    if (!first)
-        slot -= r0.slots;
-    if (slot >= r.slots)
-        return;
     constexpr uint32_t T = pvl::dmma::kUpdTile;
     const uint32_t tiles = ((r.m + T - 1) / T) * ((r.nn + T - 1) / T);
-    const uint32_t t0 = slot * r.per, t1 = min(tiles, t0 + r.per);
+    const uint32_t t0 = blockIdx.x * r.per, t1 = min(tiles, t0 + r.per);
     pvl::dmma::update_tiles<VEC>(sm, A, lda, r.row0, r.col0, r.m, r.nn, r.a_col, r.b_row, t0, t1);
 }
 
-// SMs left free while the bulk of a panel's trailing update runs on the side stream: the next
-// panel's top block, apply and pivot kernels run there meanwhile.
-constexpr int kLookaheadSms = 8;
+// CTAs (one per SM) of the update of an m x m block: the rest of the SMs is left to the next
+// panel's kernels, whose share of the work grows as the block shrinks (a share of 128, 256, 384 or
+// 768 columns' worth: n = 3072 1864, 1785, 1845, 1843 us; n = 4096 3368, 3327, 3288, 3327 us).
+constexpr uint32_t kBulkShare = 256;
+uint32_t bulk_slots(int sms, uint32_t m)
+{
+    const uint32_t free_sms = 8 + (uint32_t)sms * kBulkShare / (m + 4 * kBulkShare);
+    return (uint32_t)std::max(1, sms - (int)free_sms);
+}
+
+// Rows below the panel above which its multipliers and row block are formed in 32-wide tiles.
+constexpr uint32_t kApplyRows32Above = 2048;
 
 // A second stream and two events per thread and device for the look-ahead fork and join (a
 // stream may take part in one capture at a time: per thread, since captures here are
@@ -633,16 +526,20 @@ int side_stream(int dev, SideStream*& out)
 }
 
 // ---------------------------------------------------------------- diagonal-block inverses
-// One CTA per kRB-row block b: threads 0..63 form column c of L_bb^-1 (unit lower, forward
+// With `reject` only the blocks of panels that took the pivoting fallback (the others' inverses
+// came with their factors).  One CTA per kRB-row block b: threads 0..63 form column c of L_bb^-1 (unit lower, forward
 // substitution), threads 64..127 column c of U_bb^-1 (backward substitution), each column
 // held in registers.  A partial last block is padded with identity.  The wavefront solves
 // then apply each diagonal block as one parallel matrix-vector product.
 template <typename T>
 __global__ void __launch_bounds__(2 * kRB, 1) diag_inverse_kernel(uint32_t n, const T* __restrict__ M,
-                                                                  uint32_t lda, T* __restrict__ inv)
+                                                                  uint32_t lda, const int32_t* __restrict__ reject,
+                                                                  T* __restrict__ inv)
 {
     __shared__ T D[kRB][kRB + 1];
     const uint32_t b = blockIdx.x, r0 = b * kRB;
+    if (reject && !reject[b])
+        return;
     const uint32_t rows = min((uint32_t)kRB, n - r0);
     for (uint32_t e = threadIdx.x; e < kRB * kRB; e += blockDim.x) {
         const uint32_t r = e / kRB, c = e % kRB;
@@ -770,94 +667,100 @@ extern "C" int pvl_lu_factor(uint32_t n, double* A, uint32_t lda, int32_t* ipiv,
     SideStream* side = nullptr;
     if (int rc = side_stream(dev, side))
         return rc;
-    // 16-byte operand copies and stores need even row strides and an even width
-    const bool vec = (lda % 2 == 0) && (n % 2 == 0) && (((uintptr_t)A & 15u) == 0);
-    const void* apply_fn = vec ? (const void*)panel_apply_kernel<true> : (const void*)panel_apply_kernel<false>;
+    // 16-byte operand copies need even row strides: a matrix of odd order is factored in a copy with
+    // one (5121: 7.1 ms in place with 8-byte copies; 128-byte aligned rows; an
+    // odd last column is then copied with the padding after it).  An even order with an odd stride
+    // keeps the 8-byte copies.
+    const dim3 copy_grid(blocks_for(n, 256), std::min<uint32_t>(n, 1024));
+    double* const given = A;
+    const uint32_t given_lda = lda;
+    if (even_stride(n)) {
+        copy_matrix_kernel<<<copy_grid, 256, 0, st>>>(n, given, given_lda, w.even, even_stride(n));
+        PVL_LAUNCH_CHECK();
+        A = w.even;
+        lda = even_stride(n);
+    }
+    const bool vec = lda % 2 == 0 && ((uintptr_t)A & 15u) == 0;
+    const void* top_fn = vec ? (const void*)pvl::panel::top_factor_kernel<true>
+                             : (const void*)pvl::panel::top_factor_kernel<false>;
+    const void* apply32 = vec ? (const void*)pvl::panel::panel_apply_kernel<32, true>
+                              : (const void*)pvl::panel::panel_apply_kernel<32, false>;
+    const void* apply16 = vec ? (const void*)pvl::panel::panel_apply_kernel<16, true>
+                              : (const void*)pvl::panel::panel_apply_kernel<16, false>;
     const void* upd_fn = vec ? (const void*)dmma_update_kernel<true> : (const void*)dmma_update_kernel<false>;
+    const size_t top_smem = sizeof(pvl::panel::TopSmem);
     PVL_SMEM_OPTIN(trsm_kernel<double>, trsm_smem);
-    PVL_SMEM_OPTIN(apply_fn, kApplySmem);
+    PVL_SMEM_OPTIN(panel_pivot_kernel<double>, pivot_smem<double>(kPivotStageRows));
+    PVL_SMEM_OPTIN(top_fn, top_smem);
+    PVL_SMEM_OPTIN(apply32, pvl::panel::kApplySmem);
+    PVL_SMEM_OPTIN(apply16, pvl::panel::kApplySmem);
     PVL_SMEM_OPTIN(upd_fn, upd_smem);
-    auto update = [&](cudaStream_t s, const UpdRect& r0, const UpdRect& r1) -> int {
-        const uint32_t ctas = r0.slots + r1.slots;
-        if (ctas == 0)
-            return PVL_OK;
-        void* args[] = {(void*)&A, (void*)&lda, (void*)&r0, (void*)&r1};
-        PVL_CUDA_CHECK(cudaLaunchKernel(upd_fn, dim3(ctas), dim3(pvl::dmma::kUpdThreads), args, upd_smem, s));
-        pvl_count_launch();
-        return PVL_OK;
-    };
-    const UpdRect none{0, 0, 0, 0, 0, 0, 1, 0};
-    const uint32_t all_slots = (uint32_t)sms;  // one CTA per SM
-    const uint32_t bulk_slots = (uint32_t)std::max(1, sms - kLookaheadSms);
     int32_t* perm = ipiv + n;
     PVL_CUDA_CHECK(cudaMemsetAsync(info, 0, sizeof(int32_t), st));
     init_perm_kernel<<<blocks_for(n, 256), 256, 0, st>>>(n, perm);
     PVL_LAUNCH_CHECK();
     const uint32_t n_panels = (n + NB - 1) / NB;
     PVL_CUDA_CHECK(cudaMemsetAsync(w.reject, 0, sizeof(int32_t) * (n_panels + 1), st));
-    // Look-ahead: panel p's trailing update is split into the next panel's column and row
-    // blocks (the L shape next to this panel, on `st`) and the rest (on the side stream, on all
-    // but kLookaheadSms SMs).  Panel p + 1's top block, apply and pivot kernels touch only its
-    // own columns and row block, so they run on `st` while the rest of panel p's update is in
-    // flight; its trsm kernel (whose fallback interchanges reach every column) and everything
-    // after wait for it.
+    // Look-ahead: panel p's trailing update beyond panel p + 1 runs on the side stream, on all but
+    // a share of the SMs, while panel p + 1's diagonal block, multipliers and row block (which
+    // apply panel p's update to their own entries) run on `st`.  Panel p + 1's pivoting fallback,
+    // whose interchanges reach every column, and everything after it wait for that update.
     bool pending = false;
     for (uint32_t p = 0; p < n_panels; ++p) {
         const uint32_t k0 = p * NB;
         const uint32_t nb = std::min<uint32_t>(NB, n - k0);
         const uint32_t below = n - k0 - nb;  // nonzero only for full panels (nb == NB)
-        top_factor_kernel<<<1, kTopThreads, 0, st>>>(k0, nb, A, lda, w.top_out, w.linv, w.uinv, w.reject + p);
-        PVL_LAUNCH_CHECK();
+        const int upd = p > 0;
+        double* inv = w.inv + (size_t)p * 2 * NB * NB;
+        int32_t* rj = w.reject + p;
+        void* targs[] = {(void*)&n, (void*)&k0, (void*)&nb, (void*)&upd, (void*)&A, (void*)&lda, (void*)&w.backup,
+                         (void*)&inv, (void*)&ipiv, (void*)&rj};
+        PVL_CUDA_CHECK(cudaLaunchKernel(top_fn, dim3(1), dim3(pvl::panel::kTopThreads), targs, top_smem, st));
+        pvl_count_launch();
         if (below > 0) {
-            const uint32_t nl = blocks_for(below, kApplyRows), nu = blocks_for(below, kApplyCols);
-            double* bk = w.backup;
-            double* bkr = w.backup_row;
-            const double* li = w.linv;
-            const double* ui = w.uinv;
-            int32_t* rj = w.reject + p;
-            void* args[] = {(void*)&n, (void*)&k0, (void*)&A, (void*)&lda, (void*)&li, (void*)&ui, (void*)&bk,
-                            (void*)&bkr, (void*)&rj, (void*)&nl};
-            PVL_CUDA_CHECK(cudaLaunchKernel(apply_fn, dim3(nl + nu), dim3(pvl::dmma::kThreads), args, kApplySmem, st));
+            const uint32_t rows = below > kApplyRows32Above ? 32 : 16;
+            const uint32_t tiles = blocks_for(below, rows);
+            void* args[] = {(void*)&n, (void*)&k0, (void*)&upd, (void*)&A, (void*)&lda, (void*)&inv, (void*)&w.backup,
+                            (void*)&w.backup_row, (void*)&rj, (void*)&tiles};
+            PVL_CUDA_CHECK(cudaLaunchKernel(rows == 32 ? apply32 : apply16, dim3(2 * tiles),
+                                            dim3(pvl::panel::kApplyThreads), args, pvl::panel::kApplySmem, st));
             pvl_count_launch();
         }
-        panel_pivot_kernel<double><<<1, 1024, 0, st>>>(n, k0, nb, A, lda, w.backup, w.top_out, w.reject, w.ok, p, ipiv,
-                                                       perm, info, below > 0 ? w.backup_row : nullptr);
-        PVL_LAUNCH_CHECK();
-        if (pending) {  // the rest of the previous panel's update
+        if (pending) {  // the previous panel's update
             PVL_CUDA_CHECK(cudaEventRecord(side->join, side->s));
             PVL_CUDA_CHECK(cudaStreamWaitEvent(st, side->join, 0));
             pending = false;
         }
+        panel_pivot_kernel<double><<<1, 1024, pivot_smem<double>(n - k0), st>>>(
+            n, k0, nb, A, lda, w.backup, nullptr, w.reject, w.ok, p, ipiv, perm, info,
+            below > 0 ? w.backup_row : nullptr, kPivotStageRows);
+        PVL_LAUNCH_CHECK();
         if (n > nb) {
             trsm_kernel<double><<<blocks_for(n - nb, kTrsmCols), kTrsmCols, trsm_smem, st>>>(n, k0, nb, A, lda, w.ok, p,
                                                                                            ipiv, 1);
             PVL_LAUNCH_CHECK();
         }
-        if (below == 0)
-            continue;
-        const uint32_t base = k0 + NB;
-        if (below <= (uint32_t)pvl::dmma::kUpdTile) {  // one tile column: no look-ahead split
-            if (int rc = update(st, upd_rect(base, base, below, below, k0, all_slots), none))
-                return rc;
-            continue;
-        }
-        const uint32_t step = pvl::dmma::kUpdTile;
-        if (int rc = update(st, upd_rect(base, base, below, step, k0, all_slots),
-                            upd_rect(base, base + step, step, below - step, k0, all_slots)))
-            return rc;
+        if (below <= NB)
+            continue;  // the next panel is the last: it applies this update itself
+        const uint32_t rest = k0 + 2 * NB;
+        const UpdRect r = upd_rect(rest, rest, n - rest, n - rest, k0, bulk_slots(sms, n - rest));
         PVL_CUDA_CHECK(cudaEventRecord(side->fork, st));
         PVL_CUDA_CHECK(cudaStreamWaitEvent(side->s, side->fork, 0));
-        if (int rc = update(side->s, upd_rect(base + step, base + step, below - step, below - step, k0, bulk_slots),
-                            none))
-            return rc;
+        void* uargs[] = {(void*)&A, (void*)&lda, (void*)&r};
+        PVL_CUDA_CHECK(cudaLaunchKernel(upd_fn, dim3(r.slots), dim3(pvl::dmma::kUpdThreads), uargs, upd_smem, side->s));
+        pvl_count_launch();
         pending = true;
     }
     if (pending) {
         PVL_CUDA_CHECK(cudaEventRecord(side->join, side->s));
         PVL_CUDA_CHECK(cudaStreamWaitEvent(st, side->join, 0));
     }
-    diag_inverse_kernel<double><<<(n + kRB - 1) / kRB, 2 * kRB, 0, st>>>(n, A, lda, w.inv);
+    diag_inverse_kernel<double><<<(n + kRB - 1) / kRB, 2 * kRB, 0, st>>>(n, A, lda, w.reject, w.inv);
     PVL_LAUNCH_CHECK();
+    if (even_stride(n)) {
+        copy_matrix_kernel<<<copy_grid, 256, 0, st>>>(n, A, lda, given, given_lda);
+        PVL_LAUNCH_CHECK();
+    }
     return PVL_OK;
 }
 
@@ -1055,6 +958,7 @@ extern "C" int pvl_lu32_factor(uint32_t n, float* A, uint32_t lda, int32_t* ipiv
     float* ut = reinterpret_cast<float*>(w.backup_row);  // U12 transposed for the tensor-core updates
     const size_t trsm_smem = (size_t)(NB * (NB + 1) + NB * (kTrsmCols + 1)) * sizeof(float);
     PVL_SMEM_OPTIN(trsm_kernel<float>, trsm_smem);
+    PVL_SMEM_OPTIN(panel_pivot_kernel<float>, pivot_smem<float>(kPivotStageRows));
     int32_t* perm = ipiv + n;
     PVL_CUDA_CHECK(cudaMemsetAsync(info, 0, sizeof(int32_t), st));
     PVL_CUDA_CHECK(cudaMemsetAsync(err, 0, sizeof(int32_t), st));
@@ -1069,8 +973,8 @@ extern "C" int pvl_lu32_factor(uint32_t n, float* A, uint32_t lda, int32_t* ipiv
         const uint32_t ctas = std::max<uint32_t>(1, (below + kSlabRows - 1) / kSlabRows);
         panel_spec_kernel<float><<<ctas, 2 * kSlabRows, 0, st>>>(n, k0, nb, A, lda, backup, top_out, w.reject + p);
         PVL_LAUNCH_CHECK();
-        panel_pivot_kernel<float><<<1, 1024, 0, st>>>(n, k0, nb, A, lda, backup, top_out, w.reject, w.ok, p, ipiv,
-                                                      perm, info, nullptr);
+        panel_pivot_kernel<float><<<1, 1024, pivot_smem<float>(n - k0), st>>>(
+            n, k0, nb, A, lda, backup, top_out, w.reject, w.ok, p, ipiv, perm, info, nullptr, kPivotStageRows);
         PVL_LAUNCH_CHECK();
         if (n > nb) {
             trsm_kernel<float><<<blocks_for(n - nb, kTrsmCols), kTrsmCols, trsm_smem, st>>>(n, k0, nb, A, lda, w.ok, p,
@@ -1085,7 +989,7 @@ extern "C" int pvl_lu32_factor(uint32_t n, float* A, uint32_t lda, int32_t* ipiv
                 return r;
         }
     }
-    diag_inverse_kernel<float><<<(n + kRB - 1) / kRB, 2 * kRB, 0, st>>>(n, A, lda, inv);
+    diag_inverse_kernel<float><<<(n + kRB - 1) / kRB, 2 * kRB, 0, st>>>(n, A, lda, nullptr, inv);
     PVL_LAUNCH_CHECK();
     return PVL_OK;
 }
