@@ -368,6 +368,7 @@ class Mesh:
         return d
 
     RING_TILE = 128  # rings per tile of pvl_induction_normal_tiled
+    TILE_LINES_MAX = 3200  # lines of a tile whose values at 8 control points fit its shared memory
 
     def ring_tiles(self):
         """Per tile of RING_TILE consecutive rings: its distinct lines, and for every CSR entry
@@ -445,9 +446,17 @@ class Mesh:
         d = self.device_arrays()
         res = torch.empty((n_cp, self.n_surfaces), dtype=torch.float64, device=pos.device)
         ws, nb = Workspace.get(_lib.query("pvl_segments_workspace", self.n_lines, _lib.PVL_F64))
-        _lib.call("pvl_induction_normal", _lib.PVL_F64, self.n_points, self.n_lines, ptr(d["lines"]), ptr(pos),
-                  self.n_surfaces, ptr(d["offsets"]), ptr(d["surface_lines"]), n_cp, ptr(cps), ptr(nrm), tol,
-                  ptr(res), self.n_surfaces, ws, nb, stream_ptr())
+        if d["tile_max"] <= self.TILE_LINES_MAX:
+            # each line of a tile of rings once per control point; the other form evaluates it for
+            # every ring that it borders (4096 x 4096: 418 us)
+            _lib.call("pvl_induction_normal_tiled", self.n_points, self.n_lines, ptr(d["lines"]), ptr(pos),
+                      self.n_surfaces, ptr(d["offsets"]), ptr(d["surface_lines"]), ptr(d["tile_offsets"]),
+                      ptr(d["tile_lines"]), ptr(d["sl_local"]), d["tile_max"], n_cp, ptr(cps), ptr(nrm), tol, ptr(res),
+                      self.n_surfaces, ws, nb, stream_ptr())
+        else:  # rings of so many lines that a tile's do not fit in shared memory
+            _lib.call("pvl_induction_normal", _lib.PVL_F64, self.n_points, self.n_lines, ptr(d["lines"]), ptr(pos),
+                      self.n_surfaces, ptr(d["offsets"]), ptr(d["surface_lines"]), n_cp, ptr(cps), ptr(nrm), tol,
+                      ptr(res), self.n_surfaces, ws, nb, stream_ptr())
         return _finish(res, positions, out)
 
     def induction_matrix(self, tol, positions, control_points, out=None, line_buffer=None, /):
