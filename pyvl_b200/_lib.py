@@ -157,9 +157,17 @@ def lib() -> ctypes.CDLL:
     return _lib
 
 
+_entries: dict = {}  # entry points looked up so far
+
+
+def _entry(name: str):
+    fn = _entries[name] = getattr(lib(), name)
+    return fn
+
+
 def call(name: str, *args) -> int:
     """Call an entry point and raise on a non-zero status."""
-    rc = getattr(lib(), name)(*args)
+    rc = (_entries.get(name) or _entry(name))(*args)
     if rc != PVL_OK:
         msg = lib().pvl_last_error().decode(errors="replace")
         if rc == PVL_ERR_ARG:
@@ -170,4 +178,4 @@ def call(name: str, *args) -> int:
 
 def query(name: str, *args) -> int:
     """Call a size query (returns its value)."""
-    return int(getattr(lib(), name)(*args))
+    return int((_entries.get(name) or _entry(name))(*args))

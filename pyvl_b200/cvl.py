@@ -156,12 +156,17 @@ class Mesh:
         except TypeError as e:
             raise TypeError("Second parameter must be a sequence of sequences") from e
         counts = np.array([e.size for e in elems], np.uint32)
-        for i, e in enumerate(elems):
-            if e.size < 3:
-                raise ValueError(f"Element {i} had only {e.size} indices given (at least 3 are needed).")
-            if e.size and (e.min() < 0 or e.max() > 0xFFFFFFFF):
-                raise ValueError(f"Element {i} has an invalid point index.")
-        flat = np.ascontiguousarray(np.concatenate(elems).astype(np.uint32) if elems else np.zeros(0, np.uint32))
+        if elems:
+            every = np.concatenate(elems)
+            if counts.min() < 3 or every.min() < 0 or every.max() > 0xFFFFFFFF:
+                for i, e in enumerate(elems):  # which one
+                    if e.size < 3:
+                        raise ValueError(f"Element {i} had only {e.size} indices given (at least 3 are needed).")
+                    if e.min() < 0 or e.max() > 0xFFFFFFFF:
+                        raise ValueError(f"Element {i} has an invalid point index.")
+            flat = np.ascontiguousarray(every.astype(np.uint32))
+        else:
+            flat = np.zeros(0, np.uint32)
         total = int(flat.size)
         lines = np.zeros((max(total, 1), 2), np.uint32)
         sl = np.zeros(max(total, 1), np.uint32)

@@ -6,6 +6,7 @@ PyTorch only moves memory here; every computation is a kernel of libpvl_b200.so.
 from __future__ import annotations
 
 import ctypes
+import gc
 
 import numpy as np
 import torch
@@ -13,6 +14,8 @@ import torch
 
 def require_cuda() -> torch.device:
     """Return the current CUDA device or raise: the hot path has no CPU fallback."""
+    if torch.cuda.is_initialized() and _cur_device is not None:  # then a GPU was available
+        return torch.device("cuda", _cur_device())
     if not torch.cuda.is_available():
         raise RuntimeError("pyvl_b200 runs its kernels on a CUDA GPU (B200); no GPU is available")
     return torch.device("cuda", torch.cuda.current_device())
@@ -42,6 +45,8 @@ def to_device(a, dtype=torch.float64, device=None) -> torch.Tensor:
     """Contiguous device tensor of `dtype` (no copy when already one)."""
     dev = device or require_cuda()
     if isinstance(a, torch.Tensor):
+        if a.dtype is dtype and a.device == dev and a.is_contiguous():
+            return a
         t = a.to(device=dev, dtype=dtype)
         return t.contiguous()
     arr = np.ascontiguousarray(a)
@@ -55,6 +60,33 @@ def to_device_u32(a, device=None) -> torch.Tensor:
     return torch.from_numpy(arr.copy()).to(dev)
 
 
+def capture_graph(fn) -> torch.cuda.CUDAGraph:
+    """``fn`` (launches on fixed buffers, no host reads) captured as a CUDA graph.
+
+    torch.cuda.graph without the device-wide synchronisation, garbage collection and emptied
+    allocator cache of its entry (~1 ms a capture, more than a short run's steps take).  The
+    cyclic collector is held off instead, so that nothing it frees reaches the CUDA runtime while
+    the stream captures."""
+    g = torch.cuda.CUDAGraph()
+    cur = torch.cuda.current_stream()
+    side = torch.cuda.Stream()
+    side.wait_stream(cur)
+    collecting = gc.isenabled()
+    gc.disable()
+    try:
+        with torch.cuda.stream(side):
+            g.capture_begin()
+            try:
+                fn()
+            finally:
+                g.capture_end()
+    finally:
+        if collecting:
+            gc.enable()
+    cur.wait_stream(side)
+    return g
+
+
 class Workspace:
     """Grow-only device scratch buffer, one per (device, stream)."""
 
@@ -63,8 +95,7 @@ class Workspace:
     @classmethod
     def get(cls, nbytes: int, stream: torch.cuda.Stream | None = None) -> tuple[ctypes.c_void_p, int]:
         dev = require_cuda()
-        s = stream if stream is not None else torch.cuda.current_stream()
-        key = (dev.index, s.cuda_stream)
+        key = (dev.index, stream_ptr(stream))
         buf = cls._pool.get(key)
         nbytes = max(int(nbytes), 256)
         if buf is None or buf.numel() < nbytes:

@@ -35,7 +35,7 @@ import torch
 
 from . import _lib
 from .cvl import INVALID_ID, Mesh
-from .device import ptr, require_cuda, stream_ptr, to_device, to_device_u32
+from .device import capture_graph, ptr, require_cuda, stream_ptr, to_device, to_device_u32
 
 # pvl_gmres_status (include/pvl_b200.h) and the number of solves whose status may be in flight
 _GMRES_STATUS = np.dtype([("iterations", "<u4"), ("converged", "<u4"), ("initial_rel_residual", "<f8"),
@@ -425,9 +425,7 @@ class SolverEngine:
         entry = graphs.get(key)
         if entry is None:
             n0 = _lib.lib().pvl_launch_count()
-            g = torch.cuda.CUDAGraph()
-            with torch.cuda.graph(g):
-                fn()
+            g = capture_graph(fn)
             entry = (g, int(_lib.lib().pvl_launch_count() - n0))
             graphs[key] = entry
         entry[0].replay()
@@ -1030,10 +1028,7 @@ class MixedSolverEngine(SolverEngine):
             return
         g = self.graphs.get(key)
         if g is None:
-            g = torch.cuda.CUDAGraph()
-            with torch.cuda.graph(g):
-                fn()
-            self.graphs[key] = g
+            g = self.graphs[key] = capture_graph(fn)
         g.replay()
 
     def _gmres_start(self) -> None:
