@@ -134,7 +134,8 @@ __global__ void __launch_bounds__(128) batched_ring_kernel(const RingJob* __rest
 // tile) are evaluated at the CTA's control points into shared memory, n_i . u_l(cp_i), and
 // each thread sums its ring's signed entries (sl_local: each CSR entry's position in its
 // tile's list), in CSR order.  Adjacent rings share lines, so a quad mesh needs ~0.57 line
-// evaluations per (point, ring line) instead of one.
+// evaluations per (point, ring line) instead of one.  Lines and sums as in ring_tile_kernel
+// (induction.cu): 64 wings of 128 to 2048 rings, 716 -> 529 us.
 // FOLD (implicit wake blocks): the block is not stored; the value of control point i and
 // first-row ring j (shedding line shed = J.ring_begin + j) is folded straight into the case's
 // system matrix, A[i, adj[2 shed + 1]] -= v and A[i, adj[2 shed]] += v (out_begin / ld = the
@@ -149,9 +150,12 @@ __global__ void __launch_bounds__(128) batched_ring_tile_kernel(
     uint32_t n_lines, const Segment<double>* __restrict__ seg, const double* __restrict__ cps,
     const double* __restrict__ nrm, double tol2, const uint32_t* __restrict__ fold_adj, double* __restrict__ out)
 {
-    extern __shared__ double sV[];  // [CPB][tile_stride]
+    extern __shared__ double sV[];  // [CPB][tile_stride + 1]: a point's lines, then 0
+    const uint32_t pitch = tile_stride + 1;
     __shared__ uint32_t s_item;
-    __shared__ double s_p[CPB][3], s_n[CPB][3];
+    __shared__ __align__(16) double s_pn[CPB][6];  // control point, normal
+    if (threadIdx.x < CPB)
+        sV[threadIdx.x * pitch + tile_stride] = 0.0;
     for (;;) {
         if (threadIdx.x == 0)
             s_item = atomicAdd(counter, 1u);
@@ -169,14 +173,14 @@ __global__ void __launch_bounds__(128) batched_ring_tile_kernel(
         if (threadIdx.x < CPB * 3) {
             const uint32_t q = threadIdx.x / 3, c = threadIdx.x % 3;
             const bool ok = (int)q < nq;
-            s_p[q][c] = ok ? cps[3 * (size_t)(J.cp_begin + i0 + q) + c] : 0.0;
-            s_n[q][c] = ok ? nrm[3 * (size_t)(J.cp_begin + i0 + q) + c] : 0.0;
+            s_pn[q][c] = ok ? cps[3 * (size_t)(J.cp_begin + i0 + q) + c] : 0.0;
+            s_pn[q][3 + c] = ok ? nrm[3 * (size_t)(J.cp_begin + i0 + q) + c] : 0.0;
         }
         __syncthreads();
         const uint32_t t = job_tile[jb] + ct;
         const uint32_t L0 = tile_off[t], nl = min(tile_off[t + 1] - L0, tile_stride);
-        for (uint32_t l = threadIdx.x; l < nl; l += 128) {
-            const uint32_t g = tile_lines[L0 + l];
+        for (uint32_t l = threadIdx.x; (l & ~31u) < nl; l += 128) {  // whole warps
+            const uint32_t g = l < nl ? tile_lines[L0 + l] : n_lines;
             Segment<double> sg;
             if (g < n_lines) {
                 sg = seg[g];
@@ -184,11 +188,14 @@ __global__ void __launch_bounds__(128) batched_ring_tile_kernel(
                 sg.r1x = sg.r1y = sg.r1z = sg.dx = sg.dy = sg.dz = 0.0;
                 sg.len = sg.len2 = sg.gamma = sg.glen = sg.pad0 = sg.pad1 = 0.0;
             }
-#pragma unroll 4
-            for (int q = 0; q < nq; ++q) {
-                Vec3<double> acc{0.0, 0.0, 0.0};
-                pvl::segment_induction<double, false, true>(sg, s_p[q][0], s_p[q][1], s_p[q][2], tol2, 1.0, acc);
-                sV[q * tile_stride + l] = acc.x * s_n[q][0] + acc.y * s_n[q][1] + acc.z * s_n[q][2];
+#pragma unroll 1
+            for (int q = 0; q < nq; q += 2) {  // points past nq: zeros, never read
+                double v[2];
+                pvl::segment_normal_values<2>(sg, &s_pn[q], tol2, v);
+                if (l < nl) {
+                    sV[q * pitch + l] = v[0];
+                    sV[(q + 1) * pitch + l] = v[1];
+                }
             }
         }
         __syncthreads();
@@ -196,19 +203,26 @@ __global__ void __launch_bounds__(128) batched_ring_tile_kernel(
         if (j < J.n_rings) {
             const uint32_t r = J.ring_begin + j;
             pvl::RingEntries re;
-            re.load(sl, sl_local, off[r], off[r + 1]);
-            for (int q = 0; q < nq; ++q) {
-                const double v = re.sum(sV + q * tile_stride, tile_stride, sl, sl_local);
-                if (FOLD) {
-                    double* arow = out + J.out_begin + (size_t)(i0 + q) * J.ld;
-                    const uint32_t a1 = fold_adj[2 * (size_t)r + 1], a0 = fold_adj[2 * (size_t)r];
-                    if (a1 != PVL_INVALID && a1 < J.ld)
-                        arow[a1] -= v;
-                    if (a0 != PVL_INVALID && a0 < J.ld)
-                        arow[a0] += v;
-                } else {
-                    out[J.out_begin + (size_t)(i0 + q) * J.ld + j] = v;
+            re.load(sl, sl_local, off[r], off[r + 1], tile_stride);
+            double* o = out + J.out_begin + (size_t)i0 * J.ld + (FOLD ? 0 : j);
+            const double* row = sV;
+            if (FOLD) {
+                const uint32_t a1 = fold_adj[2 * (size_t)r + 1], a0 = fold_adj[2 * (size_t)r];
+                const bool has1 = a1 != PVL_INVALID && a1 < J.ld, has0 = a0 != PVL_INVALID && a0 < J.ld;
+                for (int q = 0; q < nq; ++q, o += J.ld, row += pitch) {
+                    const double v = re.sum(row, tile_stride, sl, sl_local);
+                    if (has1)
+                        o[a1] -= v;
+                    if (has0)
+                        o[a0] += v;
                 }
+            } else if (re.few()) {
+#pragma unroll 4
+                for (int q = 0; q < nq; ++q, o += J.ld, row += pitch)
+                    *o = re.sum_few(row);
+            } else {
+                for (int q = 0; q < nq; ++q, o += J.ld, row += pitch)
+                    *o = re.sum(row, tile_stride, sl, sl_local);
             }
         }
         __syncthreads();
@@ -728,8 +742,8 @@ int launch_ring_tiled(const void* jobs, const uint32_t* job_item, uint32_t n_job
                       uint32_t tile_stride, uint32_t n_lines, const void* seg, const double* cps, const double* nrm,
                       double tol, const uint32_t* fold_adj, double* out, uint32_t n_ctas, cudaStream_t st)
 {
-    const size_t smem = (size_t)CPB * tile_stride * sizeof(double);
-    if (smem > 200 * 1024)
+    const size_t smem = (size_t)CPB * (tile_stride + 1) * sizeof(double);
+    if ((size_t)CPB * tile_stride * sizeof(double) > 200 * 1024)
         return pvl_fail(PVL_ERR_ARG, "pvl_batch_ring_matrix_tiled: %u lines in one tile x %d control points exceed "
                         "shared memory", tile_stride, CPB);
     const void* fn = fold_adj ? (const void*)batched_ring_tile_kernel<CPB, true>

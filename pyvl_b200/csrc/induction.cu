@@ -122,9 +122,12 @@ __global__ void __launch_bounds__(kRingThreads) ring_matrix_kernel(
 // ~0.57 line evaluations per (point, ring line) instead of one.  The CTA has THREADS >=
 // kRingTile threads (chosen per launch from the largest tile's line count, so that the line
 // loop's last round is not mostly idle: 292 lines take two rounds of 160 threads instead of
-// three of 128); the first kRingTile of them sum the rings.
+// three of 128); the first kRingTile of them sum the rings.  4096 x 4096: 239 -> 186 us with two
+// points per thread between votes (segment_normal_values, 239 -> 227) and sums without tests
+// (RingEntries, 227 -> 186); bound by FP64 issue (40 instructions a pair, 29 M pairs of full warps).
 constexpr int kRingTile = 128;
-constexpr int kTileCPB = 8;   // control points per CTA (8: 231 us, 16: 272 us on the 4096-ring body)
+constexpr int kTileNQ = 2;    // points a thread works together (4096 rings and points: 1: 194 us, 2: 186, 4: 213)
+constexpr int kTileCPB = 8;   // control points per CTA (8: 186 us, 16: 185 us; 28.7 and 33.3 us for 1280 rings)
 
 template <int THREADS>
 __global__ void __launch_bounds__(THREADS) ring_tile_kernel(uint32_t n_surfaces, const uint32_t* __restrict__ off,
@@ -138,32 +141,37 @@ __global__ void __launch_bounds__(THREADS) ring_tile_kernel(uint32_t n_surfaces,
                                                               const double* __restrict__ normals, double tol2,
                                                               double* __restrict__ out, uint32_t ld)
 {
-    extern __shared__ double sV[];  // [kTileCPB][tile_stride]
-    __shared__ double s_p[kTileCPB][3], s_n[kTileCPB][3];
+    extern __shared__ double sV[];  // [kTileCPB][tile_stride + 1]: a point's lines, then 0
+    const uint32_t pitch = tile_stride + 1;
+    __shared__ __align__(16) double s_pn[kTileCPB][6];  // control point, normal
     const uint32_t tile = blockIdx.x, i0 = blockIdx.y * kTileCPB;
     if (threadIdx.x < kTileCPB * 3) {
         const uint32_t c = threadIdx.x / 3, e = threadIdx.x % 3;
         const bool ok = i0 + c < n_cp;
-        s_p[c][e] = ok ? cps[3 * (size_t)(i0 + c) + e] : 0.0;
-        s_n[c][e] = ok ? normals[3 * (size_t)(i0 + c) + e] : 0.0;
+        s_pn[c][e] = ok ? cps[3 * (size_t)(i0 + c) + e] : 0.0;
+        s_pn[c][3 + e] = ok ? normals[3 * (size_t)(i0 + c) + e] : 0.0;
+        if (e == 0)
+            sV[c * pitch + tile_stride] = 0.0;
     }
     __syncthreads();
     const uint32_t L0 = tile_off[tile], nl = tile_off[tile + 1] - L0;
-    for (uint32_t l = threadIdx.x; l < nl; l += THREADS) {
-        const uint32_t g = tile_lines[L0 + l];
-        const bool ok = g < n_lines;
+    for (uint32_t l = threadIdx.x; (l & ~31u) < nl; l += THREADS) {  // whole warps
+        const uint32_t g = l < nl ? tile_lines[L0 + l] : n_lines;
         Segment<double> sg;
-        if (ok) {
+        if (g < n_lines) {
             sg = seg[g];
         } else {
             sg.r1x = sg.r1y = sg.r1z = sg.dx = sg.dy = sg.dz = 0.0;
             sg.len = sg.len2 = sg.gamma = sg.glen = sg.pad0 = sg.pad1 = 0.0;
         }
-#pragma unroll  // all 8 control points: 232 vs 236 us for the body (unroll 4), no spills
-        for (int q = 0; q < kTileCPB; ++q) {
-            Vec3<double> acc{0.0, 0.0, 0.0};
-            pvl::segment_induction<double, false, true>(sg, s_p[q][0], s_p[q][1], s_p[q][2], tol2, 1.0, acc);
-            sV[q * tile_stride + l] = acc.x * s_n[q][0] + acc.y * s_n[q][1] + acc.z * s_n[q][2];
+#pragma unroll 1
+        for (int q = 0; q < kTileCPB; q += kTileNQ) {
+            double v[kTileNQ];
+            pvl::segment_normal_values<kTileNQ>(sg, &s_pn[q], tol2, v);
+            if (l < nl)
+#pragma unroll
+                for (int u = 0; u < kTileNQ; ++u)
+                    sV[(q + u) * pitch + l] = v[u];
         }
     }
     __syncthreads();
@@ -171,11 +179,16 @@ __global__ void __launch_bounds__(THREADS) ring_tile_kernel(uint32_t n_surfaces,
     if (threadIdx.x >= kRingTile || j >= n_surfaces)
         return;
     pvl::RingEntries re;
-    re.load(sl, sl_local, off[j], off[j + 1]);
-    for (int q = 0; q < kTileCPB; ++q) {
-        if (i0 + q >= n_cp)
-            break;
-        out[(size_t)(i0 + q) * ld + j] = re.sum(sV + q * tile_stride, tile_stride, sl, sl_local);
+    re.load(sl, sl_local, off[j], off[j + 1], tile_stride);
+    double* o = out + (size_t)i0 * ld + j;
+    const double* row = sV;
+    if (re.few() && i0 + kTileCPB <= n_cp) {
+#pragma unroll
+        for (int q = 0; q < kTileCPB; ++q, o += ld, row += pitch)
+            *o = re.sum_few(row);
+    } else {
+        for (uint32_t q = 0; q < (uint32_t)kTileCPB && i0 + q < n_cp; ++q, o += ld, row += pitch)
+            *o = re.sum(row, tile_stride, sl, sl_local);
     }
 }
 
@@ -861,15 +874,17 @@ extern "C" int pvl_induction_normal_tiled(uint32_t n_points, uint32_t n_lines, c
         return pvl_fail(PVL_ERR_ARG, "pvl_induction_normal_tiled: ld < n_surfaces");
     if (ws_bytes < pvl_segments_workspace(n_lines, PVL_F64))
         return pvl_fail(PVL_ERR_ALLOC, "pvl_induction_normal_tiled: workspace too small");
-    const size_t smem = (size_t)kTileCPB * max_tile_lines * sizeof(double);
-    if (smem > 200 * 1024)
+    if ((size_t)kTileCPB * max_tile_lines * sizeof(double) > 200 * 1024)
         return pvl_fail(PVL_ERR_ARG, "pvl_induction_normal_tiled: %u lines in one ring tile exceed shared memory",
                         max_tile_lines);
+    const size_t smem = (size_t)kTileCPB * (max_tile_lines + 1) * sizeof(double);
+    dim3 grid(blocks_for(n_surfaces, kRingTile), blocks_for(n_cp, kTileCPB));
+    if (grid.y > 65535)
+        return pvl_fail(PVL_ERR_ARG, "pvl_induction_normal_tiled: too many points (%u)", n_cp);
     cudaStream_t st = (cudaStream_t)stream;
     auto* seg = static_cast<Segment<double>*>(ws);
     if (int r = prep_segments<double>(n_points, n_lines, lines, positions, nullptr, tol, seg, st))
         return r;
-    dim3 grid((n_surfaces + kRingTile - 1) / kRingTile, (n_cp + kTileCPB - 1) / kTileCPB);
     switch (ring_tile_threads(max_tile_lines)) {
     case 160:
         return launch_ring_tile<160>(grid, smem, st, n_surfaces, offsets, surface_lines, sl_local, tile_offsets,

@@ -201,6 +201,66 @@ __device__ __forceinline__ void segment_induction(const Segment<T>& s, T px, T p
     acc.z += cz * mag;
 }
 
+// n_q . u(p_q) of one segment at NQ points, pn[q] = the point and its normal (tiled ring matrices: a
+// lane holds a line, so all 32 lanes of a warp call it together, lanes without a line with the
+// disabled segment d = 0).  segment_induction's arithmetic up to the series argument w and its tiers
+// (the normal enters as (c . n) mag, one rounding less), but the NQ points are worked without a
+// branch between them and one vote decides the tier of all of them: a pair costs about 40 FP64
+// instructions and 15 others, where one call per point took 90 others (per-point votes inside
+// branches, scalar loads of the point) and was bound by instruction issue.  Pairs that need more
+// than eight terms on any lane (5 % of the warps' pairs on a 4096-ring wing, 2 % have a near pair)
+// take the per-lane forms.
+template <int NQ>
+__device__ __forceinline__ void segment_normal_values(const Segment<double>& s, const double (*__restrict__ pn)[6],
+                                                      double tol2, double (&v)[NQ])
+{
+    using F = FarSeries<double>;
+    double r[NQ], w[NQ];
+    double hs[NQ], xs[NQ];
+    int worst = 0;  // high word of the largest w; the largest int where x is not positive
+    bool cut[NQ];
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+        const double2 p01 = *reinterpret_cast<const double2*>(&pn[q][0]);
+        const double2 p2n = *reinterpret_cast<const double2*>(&pn[q][2]);
+        const double2 n12 = *reinterpret_cast<const double2*>(&pn[q][4]);
+        const double ax = p01.x - s.r1x, ay = p01.y - s.r1y, az = p2n.x - s.r1z;
+        const double t1 = s.dx * ax + s.dy * ay + s.dz * az;
+        const double cx = ay * s.dz - az * s.dy, cy = az * s.dx - ax * s.dz, cz = ax * s.dy - ay * s.dx;
+        const double h = cx * cx + cy * cy + cz * cz;
+        v[q] = cx * p2n.y + cy * n12.x + cz * n12.y;
+        const double x = h + t1 * (t1 - s.len);
+        r[q] = F::rcp(x);
+        w[q] = h * s.len2 * (r[q] * r[q]);
+        hs[q] = h;
+        xs[q] = x;
+        cut[q] = lt_nn(h, tol2);
+        const int m = pos_hi(x) ? hi32(w[q]) : 0x7FFFFFFF;
+        worst = max(worst, cut[q] ? 0 : m);
+    }
+    if (__any_sync(0xFFFFFFFFu, worst > hi32(0.01))) {
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) {
+            double mag;
+            if (pos_hi(xs[q]) && le_hi(w[q], F::kW)) {
+                mag = -s.len * r[q] * F::sum_tier<16>(w[q]);
+            } else {
+                const double rh = rsqrt(hs[q]);
+                mag = atan2(-(hs[q] * rh) * s.len, xs[q]) * rh;
+            }
+            v[q] = cut[q] ? 0.0 : v[q] * mag;
+        }
+    } else if (__any_sync(0xFFFFFFFFu, worst > hi32(1e-4))) {
+#pragma unroll
+        for (int q = 0; q < NQ; ++q)
+            v[q] = cut[q] ? 0.0 : v[q] * (-s.len * r[q] * F::sum_tier<8>(w[q]));
+    } else {
+#pragma unroll
+        for (int q = 0; q < NQ; ++q)
+            v[q] = cut[q] ? 0.0 : v[q] * (-s.len * r[q] * F::sum_tier<4>(w[q]));
+    }
+}
+
 // The segments of one ring (its entries k0 .. k1 of the ring -> line CSR) held in registers,
 // so that a thread evaluating the ring at many control points loads them once.  Rings of up
 // to kMax lines are cached (quads and triangles); larger rings fall back to loading per point.
@@ -262,43 +322,53 @@ struct RingSegments {
 // registers for rings of up to kMax lines (quads and triangles), so that summing the ring at
 // every control point of a CTA reads its CSR entries once; larger rings read them per point.
 // sum() adds +-row[e] in CSR order (the reference's order); an entry at or past `stride` adds 0.
+// row[stride] holds 0: an absent entry of a short ring points there and a reversed line flips the
+// sign bit, so that a point costs four loads, four integer operations and four additions (with a
+// test and a selection for each entry instead, the sums of quads took as many instructions as the
+// evaluation of their lines).
 struct RingEntries {
     static constexpr int kMax = 4;
     uint32_t e[kMax];
-    bool neg[kMax];
+    int flip[kMax];
     uint32_t k0, k1;
 
     __device__ __forceinline__ void load(const uint32_t* __restrict__ sl, const uint32_t* __restrict__ sl_local,
-                                         uint32_t k0_, uint32_t k1_)
+                                         uint32_t k0_, uint32_t k1_, uint32_t stride)
     {
         k0 = k0_;
         k1 = k1_;
 #pragma unroll
         for (int u = 0; u < kMax; ++u) {
             const bool ok = k1 - k0 <= (uint32_t)kMax && k0 + u < k1;
-            e[u] = ok ? sl_local[k0 + u] : 0u;
-            neg[u] = ok ? PVL_REV(sl[k0 + u]) != 0 : false;
+            e[u] = ok ? min(sl_local[k0 + u], stride) : stride;
+            flip[u] = ok && PVL_REV(sl[k0 + u]) ? (int)0x80000000 : 0;
         }
+    }
+
+    __device__ __forceinline__ bool few() const { return k1 - k0 <= (uint32_t)kMax; }
+
+    // rings of up to kMax lines
+    __device__ __forceinline__ double sum_few(const double* __restrict__ row) const
+    {
+        double v = 0.0;
+#pragma unroll
+        for (int u = 0; u < kMax; ++u) {
+            const double x = row[e[u]];
+            v += __hiloint2double(__double2hiint(x) ^ flip[u], __double2loint(x));
+        }
+        return v;
     }
 
     __device__ __forceinline__ double sum(const double* __restrict__ row, uint32_t stride,
                                           const uint32_t* __restrict__ sl, const uint32_t* __restrict__ sl_local) const
     {
+        if (few())
+            return sum_few(row);
         double v = 0.0;
-        if (k1 - k0 <= (uint32_t)kMax) {
-#pragma unroll
-            for (int u = 0; u < kMax; ++u) {
-                if (k0 + u < k1) {
-                    const double x = e[u] < stride ? row[e[u]] : 0.0;
-                    v += neg[u] ? -x : x;
-                }
-            }
-        } else {
-            for (uint32_t k = k0; k < k1; ++k) {
-                const uint32_t ek = sl_local[k];
-                const double x = ek < stride ? row[ek] : 0.0;
-                v += PVL_REV(sl[k]) ? -x : x;
-            }
+        for (uint32_t k = k0; k < k1; ++k) {
+            const uint32_t ek = sl_local[k];
+            const double x = ek < stride ? row[ek] : 0.0;
+            v += PVL_REV(sl[k]) ? -x : x;
         }
         return v;
     }
