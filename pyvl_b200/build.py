@@ -6,8 +6,7 @@ The library is compiled from pyvl_b200/csrc/*.cu and *.cpp with
 ``-gencode arch=compute_100a,code=sm_100a`` and lands next to this file, where the
 Python layer loads it.  nvcc cross-compiles without a GPU.  Beside it, libpvl_probe.so
 (pyvl_b200/probe: an FMA-throughput probe and test hooks) is built for benchmarks and tests;
-the product never loads it.  Extra nvcc flags (e.g. a tuning define such as
-``-DPVL_UPD_WARPS=4``) can be passed in the environment variable PVL_NVCC_FLAGS.
+the product never loads it.  Extra nvcc flags (e.g. ``-DNAME=VALUE``) can be passed in the environment variable PVL_NVCC_FLAGS.
 """
 
 from __future__ import annotations

@@ -315,8 +315,7 @@ __global__ void __launch_bounds__(THREADS) batched_sweep_kernel(const SweepJob* 
                     const pvl::SweepSeg a = s_seg[k], b = s_seg[k + 1 < cnt ? k + 1 : kSegTile];
                     const pvl::SweepGeo ga = pvl::sweep_geo(a, px[0], py[0], pz[0]);
                     const pvl::SweepGeo gb = pvl::sweep_geo(b, px[0], py[0], pz[0]);
-                    pvl::sweep_add(a, ga, tol2, acc[0]);
-                    pvl::sweep_add(b, gb, tol2, acc[0]);
+                    pvl::sweep_add2(a, ga, b, gb, tol2, acc[0], acc[0]);
                 }
             } else {
 #pragma unroll 1

@@ -454,46 +454,46 @@ __global__ void __launch_bounds__(kTrsmCols, 1) trsm_kernel(uint32_t n, uint32_t
 
 // One rectangle of the trailing update A22 -= L21 U12: C = rows row0 .. row0 + m, columns
 // col0 .. col0 + nn; A = the panel's L21 (columns a_col ..) on C's rows, B = its U12 (rows
-// b_row ..) on C's columns.  `slots` runs of `per` 64 x 64 tiles.
+// b_row ..) on C's columns.  `ctas` CTAs, each group of a CTA a run of `per` 64 x 64 tiles.
 struct UpdRect {
-    uint32_t row0, col0, m, nn, a_col, b_row, per, slots;
+    uint32_t row0, col0, m, nn, a_col, b_row, per, ctas;
 };
 
-UpdRect upd_rect(uint32_t row0, uint32_t col0, uint32_t m, uint32_t nn, uint32_t k0, uint32_t max_slots)
+UpdRect upd_rect(uint32_t row0, uint32_t col0, uint32_t m, uint32_t nn, uint32_t k0, uint32_t max_ctas)
 {
     const uint32_t tiles = blocks_for(m, pvl::dmma::kUpdTile) * blocks_for(nn, pvl::dmma::kUpdTile);
-    UpdRect r{row0, col0, m, nn, k0, k0, 0, 0};
-    r.per = tiles ? blocks_for(tiles, std::max(1u, max_slots)) : 1;
-    r.slots = blocks_for(tiles, r.per);
+    UpdRect r{row0, col0, m, nn, k0, k0, 1, tiles};
+    if (tiles > max_ctas) {  // fewer tiles than CTAs: one each, on SMs of their own
+        r.per = blocks_for(tiles, pvl::dmma::kUpdGroups * max_ctas);
+        r.ctas = blocks_for(blocks_for(tiles, r.per), pvl::dmma::kUpdGroups);
+    }
     return r;
 }
 
-// One CTA per SM, each a run of tiles (dmma.cuh update_tiles: C and A blocks stream into shared
-// memory one tile ahead of the MMAs), in column-major order.
+// One CTA per SM, each of its two groups a run of tiles in column-major order (dmma.cuh update_tiles).
 template <bool VEC>
 __global__ void __launch_bounds__(pvl::dmma::kUpdThreads, 1) dmma_update_kernel(double* __restrict__ A, uint32_t lda,
                                                                             UpdRect r)
 {
     extern __shared__ __align__(16) double upd_smem[];
-    auto& sm = *reinterpret_cast<pvl::dmma::UpdSmem*>(upd_smem);
-    constexpr uint32_t T = pvl::dmma::kUpdTile;
+    auto* sm = reinterpret_cast<pvl::dmma::UpdSmem*>(upd_smem);
+    constexpr uint32_t T = pvl::dmma::kUpdTile, G = pvl::dmma::kUpdGroupThreads;
     const uint32_t tiles = ((r.m + T - 1) / T) * ((r.nn + T - 1) / T);
-    const uint32_t t0 = blockIdx.x * r.per, t1 = min(tiles, t0 + r.per);
-    pvl::dmma::update_tiles<VEC>(sm, A, lda, r.row0, r.col0, r.m, r.nn, r.a_col, r.b_row, t0, t1);
+    const uint32_t group = threadIdx.x / G, run = blockIdx.x + group * gridDim.x;
+    const uint32_t t0 = min(tiles, run * r.per), t1 = min(tiles, t0 + r.per);
+    pvl::dmma::update_tiles<VEC>(sm[group], (int)group, threadIdx.x % G, A, lda, r.row0, r.col0, r.m, r.nn, r.a_col,
+                                 r.b_row, t0, t1);
 }
 
 // CTAs (one per SM) of the update of an m x m block: the rest of the SMs is left to the next
-// panel's kernels, whose share of the work grows as the block shrinks (a share of 128, 256, 384 or
-// 768 columns' worth: n = 3072 1864, 1785, 1845, 1843 us; n = 4096 3368, 3327, 3288, 3327 us).
+// panel's kernels, whose share of the work grows as the block shrinks (a share of 256, 400 or 600
+// columns' worth: n = 3072 1776, 1786, 1796 us; n = 4096 3127, 3136, 3163; 128: 70 us more).
 constexpr uint32_t kBulkShare = 256;
-uint32_t bulk_slots(int sms, uint32_t m)
+uint32_t bulk_ctas(int sms, uint32_t m)
 {
     const uint32_t free_sms = 8 + (uint32_t)sms * kBulkShare / (m + 4 * kBulkShare);
     return (uint32_t)std::max(1, sms - (int)free_sms);
 }
-
-// Rows below the panel above which its multipliers and row block are formed in 32-wide tiles.
-constexpr uint32_t kApplyRows32Above = 2048;
 
 // A second stream and two events per thread and device for the look-ahead fork and join (a
 // stream may take part in one capture at a time: per thread, since captures here are
@@ -660,7 +660,7 @@ extern "C" int pvl_lu_factor(uint32_t n, double* A, uint32_t lda, int32_t* ipiv,
     cudaStream_t st = (cudaStream_t)stream;
     LuWs w = carve(ws, n);
     const size_t trsm_smem = (size_t)(NB * (NB + 1) + NB * (kTrsmCols + 1)) * sizeof(double);
-    const size_t upd_smem = sizeof(pvl::dmma::UpdSmem);
+    const size_t upd_smem = pvl::dmma::kUpdGroups * sizeof(pvl::dmma::UpdSmem);
     int dev = 0, sms = 0;
     PVL_CUDA_CHECK(cudaGetDevice(&dev));
     PVL_CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
@@ -683,17 +683,14 @@ extern "C" int pvl_lu_factor(uint32_t n, double* A, uint32_t lda, int32_t* ipiv,
     const bool vec = lda % 2 == 0 && ((uintptr_t)A & 15u) == 0;
     const void* top_fn = vec ? (const void*)pvl::panel::top_factor_kernel<true>
                              : (const void*)pvl::panel::top_factor_kernel<false>;
-    const void* apply32 = vec ? (const void*)pvl::panel::panel_apply_kernel<32, true>
-                              : (const void*)pvl::panel::panel_apply_kernel<32, false>;
-    const void* apply16 = vec ? (const void*)pvl::panel::panel_apply_kernel<16, true>
-                              : (const void*)pvl::panel::panel_apply_kernel<16, false>;
+    const void* apply_fn = vec ? (const void*)pvl::panel::panel_apply_kernel<true>
+                               : (const void*)pvl::panel::panel_apply_kernel<false>;
     const void* upd_fn = vec ? (const void*)dmma_update_kernel<true> : (const void*)dmma_update_kernel<false>;
     const size_t top_smem = sizeof(pvl::panel::TopSmem);
     PVL_SMEM_OPTIN(trsm_kernel<double>, trsm_smem);
     PVL_SMEM_OPTIN(panel_pivot_kernel<double>, pivot_smem<double>(kPivotStageRows));
     PVL_SMEM_OPTIN(top_fn, top_smem);
-    PVL_SMEM_OPTIN(apply32, pvl::panel::kApplySmem);
-    PVL_SMEM_OPTIN(apply16, pvl::panel::kApplySmem);
+    PVL_SMEM_OPTIN(apply_fn, pvl::panel::kApplySmem);
     PVL_SMEM_OPTIN(upd_fn, upd_smem);
     int32_t* perm = ipiv + n;
     PVL_CUDA_CHECK(cudaMemsetAsync(info, 0, sizeof(int32_t), st));
@@ -718,12 +715,11 @@ extern "C" int pvl_lu_factor(uint32_t n, double* A, uint32_t lda, int32_t* ipiv,
         PVL_CUDA_CHECK(cudaLaunchKernel(top_fn, dim3(1), dim3(pvl::panel::kTopThreads), targs, top_smem, st));
         pvl_count_launch();
         if (below > 0) {
-            const uint32_t rows = below > kApplyRows32Above ? 32 : 16;
-            const uint32_t tiles = blocks_for(below, rows);
+            const uint32_t tiles = blocks_for(below, pvl::panel::kApplyRows);
             void* args[] = {(void*)&n, (void*)&k0, (void*)&upd, (void*)&A, (void*)&lda, (void*)&inv, (void*)&w.backup,
                             (void*)&w.backup_row, (void*)&rj, (void*)&tiles};
-            PVL_CUDA_CHECK(cudaLaunchKernel(rows == 32 ? apply32 : apply16, dim3(2 * tiles),
-                                            dim3(pvl::panel::kApplyThreads), args, pvl::panel::kApplySmem, st));
+            PVL_CUDA_CHECK(cudaLaunchKernel(apply_fn, dim3(2 * tiles), dim3(pvl::panel::kApplyThreads), args,
+                                            pvl::panel::kApplySmem, st));
             pvl_count_launch();
         }
         if (pending) {  // the previous panel's update
@@ -743,11 +739,11 @@ extern "C" int pvl_lu_factor(uint32_t n, double* A, uint32_t lda, int32_t* ipiv,
         if (below <= NB)
             continue;  // the next panel is the last: it applies this update itself
         const uint32_t rest = k0 + 2 * NB;
-        const UpdRect r = upd_rect(rest, rest, n - rest, n - rest, k0, bulk_slots(sms, n - rest));
+        const UpdRect r = upd_rect(rest, rest, n - rest, n - rest, k0, bulk_ctas(sms, n - rest));
         PVL_CUDA_CHECK(cudaEventRecord(side->fork, st));
         PVL_CUDA_CHECK(cudaStreamWaitEvent(side->s, side->fork, 0));
         void* uargs[] = {(void*)&A, (void*)&lda, (void*)&r};
-        PVL_CUDA_CHECK(cudaLaunchKernel(upd_fn, dim3(r.slots), dim3(pvl::dmma::kUpdThreads), uargs, upd_smem, side->s));
+        PVL_CUDA_CHECK(cudaLaunchKernel(upd_fn, dim3(r.ctas), dim3(pvl::dmma::kUpdThreads), uargs, upd_smem, side->s));
         pvl_count_launch();
         pending = true;
     }

@@ -399,11 +399,14 @@ __global__ void __launch_bounds__(kTopThreads, 1) top_factor_kernel(uint32_t n, 
 // the rest: R columns of the panel's row block,
 //   A12 := L11^-1 (A12 - L[p, p-1] U[p-1, .]).
 // 4 warps; the updated operand goes through shared memory between the two products, and to the
-// backup.  R = 32 while there are tiles enough for the SMs, 16 beyond (half the chain per CTA).
+// backup.  R = 16 at every size: the shortest chain per CTA, and the few SMs that the bulk update
+// leaves are shared most evenly (n = 2048: 957 us; 32 rows above 1024 rows 982, 64 above 1600 1008;
+// n = 4096: 3108, 3187, 3278).
+constexpr int kApplyRows = 16;
 constexpr int kApplyThreads = 128;
 constexpr size_t kApplySmem = (size_t)3 * NB * kPad * sizeof(double);
 
-template <int R, bool VEC>
+template <bool VEC>
 __global__ void __launch_bounds__(kApplyThreads, 2) panel_apply_kernel(uint32_t n, uint32_t k0, int update,
                                                                        double* __restrict__ A, uint32_t lda,
                                                                        const double* __restrict__ inv,
@@ -411,7 +414,7 @@ __global__ void __launch_bounds__(kApplyThreads, 2) panel_apply_kernel(uint32_t 
                                                                        double* __restrict__ backup_row,
                                                                        int32_t* __restrict__ reject, uint32_t n_ltiles)
 {
-    static_assert(R == 16 || R == 32, "tile rows");
+    constexpr int R = kApplyRows;
     extern __shared__ __align__(16) double apply_smem[];
     double* s0 = apply_smem;              // L: R x 64 rows / U: 64 x 64 of L[p, p-1]
     double* s1 = s0 + NB * kPad;          // U[p-1, .] (64 x 64 / 64 x R)
@@ -424,26 +427,26 @@ __global__ void __launch_bounds__(kApplyThreads, 2) panel_apply_kernel(uint32_t 
     const uint32_t cnt = min((uint32_t)R, n - e0);
     bool bad = false;
     if (lower) {
-        constexpr int WN = R == 32 ? 2 : 4, NT = 8 / WN;  // warps along the 64 columns
-        const uint32_t wm0 = (warp / WN) * 16, wn0 = (warp % WN) * (8 * NT);
+        constexpr int NT = 2;  // every warp: 16 rows x 16 columns
+        const uint32_t wn0 = warp * 16;
         double acc[1][NT][4];
         if (update) {
             dmma::stage_tile<R, NB, VEC, kApplyThreads>(s0, A, lda, e0, e0 + cnt, k0 - NB, k0, tid);
             dmma::stage_tile<NB, NB, VEC, kApplyThreads>(s1, A, lda, k0 - NB, k0, k0, base, tid);
         }
         dmma::stage_tile<NB, NB, true, kApplyThreads>(s2, inv + NB * NB, NB, 0, NB, 0, NB, tid);
-        load_neg<1, NT, VEC>(acc, A + (size_t)e0 * lda + k0, lda, wm0, wn0, cnt, NB, g, t4);
+        load_neg<1, NT, VEC>(acc, A + (size_t)e0 * lda + k0, lda, 0, wn0, cnt, NB, g, t4);
         dmma::cp_async_wait_all();
         __syncthreads();
         if (update) {
-            mma_k64<1, NT>(acc, s0 + wm0 * kPad, s1 + wn0, g, t4);
+            mma_k64<1, NT>(acc, s0, s1 + wn0, g, t4);
             __syncthreads();
         }
 #pragma unroll
         for (int j = 0; j < NT; ++j)
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-                const uint32_t r = wm0 + g + 8 * h, c = wn0 + 8 * j + 2 * t4;
+                const uint32_t r = g + 8 * h, c = wn0 + 8 * j + 2 * t4;
                 const double2 v = make_double2(-acc[0][j][2 * h], -acc[0][j][2 * h + 1]);
                 *reinterpret_cast<double2*>(s0 + r * kPad + c) = v;
                 if (r < cnt)
@@ -451,12 +454,12 @@ __global__ void __launch_bounds__(kApplyThreads, 2) panel_apply_kernel(uint32_t 
                 acc[0][j][2 * h] = acc[0][j][2 * h + 1] = 0.0;
             }
         __syncthreads();
-        mma_k64<1, NT>(acc, s0 + wm0 * kPad, s2 + wn0, g, t4);
+        mma_k64<1, NT>(acc, s0, s2 + wn0, g, t4);
 #pragma unroll
         for (int j = 0; j < NT; ++j)
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-                const uint32_t r = wm0 + g + 8 * h, c = wn0 + 8 * j + 2 * t4;
+                const uint32_t r = g + 8 * h, c = wn0 + 8 * j + 2 * t4;
                 if (r >= cnt)
                     continue;
                 const double v0 = acc[0][j][2 * h], v1 = acc[0][j][2 * h + 1];

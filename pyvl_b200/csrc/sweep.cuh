@@ -78,6 +78,40 @@ __device__ __forceinline__ void sweep_add(const SweepSeg& s, const SweepGeo& g, 
     acc.z += g.cz * mag;
 }
 
+// gamma_a u_a(p_a) and gamma_b u_b(p_b) added to A and B (one accumulator, or two points'): as two
+// sweep_add calls, with the tier of both pairs of all lanes decided by one vote, so that the usual
+// eight or four terms run without a branch per pair.  Every lane of the warp calls it.
+__device__ __forceinline__ void sweep_add2(const SweepSeg& a, const SweepGeo& ga, const SweepSeg& b,
+                                           const SweepGeo& gb, double tol2, Vec3<double>& A, Vec3<double>& B)
+{
+    using F = FarSeries<double>;
+    const bool cut_a = lt_nn(ga.hsq, tol2), cut_b = lt_nn(gb.hsq, tol2);
+    const int ma = cut_a ? 0 : pos_hi(ga.x) ? hi32(ga.w) : 0x7FFFFFFF;
+    const int mb = cut_b ? 0 : pos_hi(gb.x) ? hi32(gb.w) : 0x7FFFFFFF;
+    const int worst = max(ma, mb);
+    if (__any_sync(0xFFFFFFFFu, worst > hi32(0.01))) {
+        sweep_add(a, ga, tol2, A);
+        sweep_add(b, gb, tol2, B);
+        return;
+    }
+    double fa = -a.glen * ga.r, fb = -b.glen * gb.r;
+    if (__any_sync(0xFFFFFFFFu, worst > hi32(1e-4))) {
+        fa *= F::sum_tier<8>(ga.w);
+        fb *= F::sum_tier<8>(gb.w);
+    } else {
+        fa *= F::sum_tier<4>(ga.w);
+        fb *= F::sum_tier<4>(gb.w);
+    }
+    fa = cut_a ? 0.0 : fa;
+    fb = cut_b ? 0.0 : fb;
+    A.x += ga.cx * fa;
+    A.y += ga.cy * fa;
+    A.z += ga.cz * fa;
+    B.x += gb.cx * fb;
+    B.y += gb.cy * fb;
+    B.z += gb.cz * fb;
+}
+
 // o = centroid of the CTA's valid points (0 if none), in fixed summation order, from each
 // thread's sum of its valid points (sx, sy, sz) and their count n; every thread of the CTA
 // must call it.  red: THREADS / 32 x 4 doubles of shared memory, o: 3.

@@ -1,6 +1,6 @@
 """The FP64 LU and its solve at the sizes where their tiles, copies and fallbacks meet: panel and
 row-block edges, odd orders (factored in a copy with aligned rows), row strides beyond the order
-(odd and even), the switch of the multiplier tiles from 16 to 32 rows, and rejected panels factored
+(odd and even), updates with fewer tiles than SMs and with several per group, and rejected panels factored
 in shared memory and in place.  Against scipy's LAPACK."""
 
 import numpy as np
