@@ -156,6 +156,12 @@ __device__ __forceinline__ void tiles(double* m, const int (&dst)[N], const int 
             *reinterpret_cast<double2*>(m + dst[u]) = c[u];
 }
 
+// Programmatic dependent launch (the chain's kernels may be started before the one ahead of them in
+// the stream has ended): wait until it has, its writes visible; and let the next kernel start.
+// Every kernel launched so waits before it ends, so its own end implies all earlier ones'.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_launch_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 __device__ __forceinline__ void panel_group_sync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 
 // The high word of |v|: an order on magnitudes to 2^-20, compared on the integer pipe.
@@ -181,6 +187,7 @@ __global__ void __launch_bounds__(kTopThreads, 1) top_factor_kernel(uint32_t n, 
     double* ls = m;                       // L[p, p-1] and U[p-1, p] (stride kPad), before xt and y are needed
     double* us = ls + NB * kPad;
     static_assert(sizeof(TopSmem) >= 2 * NB * kPad * sizeof(double), "the corner's operands fit");
+    grid_wait();
     if (update) {
         dmma::stage_tile<NB, NB, VEC, kTopThreads>(ls, A, lda, k0, k0 + nb, k0 - NB, k0, tid);
         dmma::stage_tile<NB, NB, VEC, kTopThreads>(us, A, lda, k0 - NB, k0, k0, k0 + nb, tid);
@@ -363,6 +370,7 @@ __global__ void __launch_bounds__(kTopThreads, 1) top_factor_kernel(uint32_t n, 
         if (warp < 4)
             panel_group_sync();
     }
+    grid_launch_next();  // panel_apply_kernel: its first product needs nothing of this block
     // the range of a pivot that pivot_rcp takes, and the limit of a multiplier (both to the high word:
     // what lies within 2^-20 of a bound takes the pivoting path, which is always right)
     const bool bad = lo <= __double2hiint(kPivotLo) || hi >= __double2hiint(kPivotHi) ||
@@ -399,7 +407,8 @@ __global__ void __launch_bounds__(kTopThreads, 1) top_factor_kernel(uint32_t n, 
 // the rest: R columns of the panel's row block,
 //   A12 := L11^-1 (A12 - L[p, p-1] U[p-1, .]).
 // 4 warps; the updated operand goes through shared memory between the two products, and to the
-// backup.  R = 16 at every size: the shortest chain per CTA, and the few SMs that the bulk update
+// backup.  The first product reads only what older panels left, so it runs before grid_wait, beside
+// the end of top_factor_kernel.  R = 16 at every size: the shortest chain per CTA, and the few SMs that the bulk update
 // leaves are shared most evenly (n = 2048: 957 us; 32 rows above 1024 rows 982, 64 above 1600 1008;
 // n = 4096: 3108, 3187, 3278).
 constexpr int kApplyRows = 16;
@@ -434,14 +443,14 @@ __global__ void __launch_bounds__(kApplyThreads, 2) panel_apply_kernel(uint32_t 
             dmma::stage_tile<R, NB, VEC, kApplyThreads>(s0, A, lda, e0, e0 + cnt, k0 - NB, k0, tid);
             dmma::stage_tile<NB, NB, VEC, kApplyThreads>(s1, A, lda, k0 - NB, k0, k0, base, tid);
         }
-        dmma::stage_tile<NB, NB, true, kApplyThreads>(s2, inv + NB * NB, NB, 0, NB, 0, NB, tid);
         load_neg<1, NT, VEC>(acc, A + (size_t)e0 * lda + k0, lda, 0, wn0, cnt, NB, g, t4);
         dmma::cp_async_wait_all();
         __syncthreads();
-        if (update) {
+        if (update)
             mma_k64<1, NT>(acc, s0, s1 + wn0, g, t4);
-            __syncthreads();
-        }
+        grid_wait();
+        dmma::stage_tile<NB, NB, true, kApplyThreads>(s2, inv + NB * NB, NB, 0, NB, 0, NB, tid);
+        __syncthreads();  // s0 is read no more
 #pragma unroll
         for (int j = 0; j < NT; ++j)
 #pragma unroll
@@ -453,6 +462,7 @@ __global__ void __launch_bounds__(kApplyThreads, 2) panel_apply_kernel(uint32_t 
                     *reinterpret_cast<double2*>(backup + (size_t)(e0 + r - k0) * NB + c) = v;
                 acc[0][j][2 * h] = acc[0][j][2 * h + 1] = 0.0;
             }
+        dmma::cp_async_wait_all();
         __syncthreads();
         mma_k64<1, NT>(acc, s0, s2 + wn0, g, t4);
 #pragma unroll
@@ -480,14 +490,14 @@ __global__ void __launch_bounds__(kApplyThreads, 2) panel_apply_kernel(uint32_t 
             dmma::stage_tile<NB, NB, VEC, kApplyThreads>(s0, A, lda, k0, base, k0 - NB, k0, tid);
             dmma::stage_tile<NB, R, VEC, kApplyThreads>(s1, A, lda, k0 - NB, k0, e0, e0 + cnt, tid);
         }
-        dmma::stage_tile<NB, NB, true, kApplyThreads>(s2, inv, NB, 0, NB, 0, NB, tid);
         load_neg<1, NT, VEC>(acc, A + (size_t)k0 * lda + e0, lda, wm0, 0, NB, cnt, g, t4);
         dmma::cp_async_wait_all();
         __syncthreads();
-        if (update) {
+        if (update)
             mma_k64<1, NT>(acc, s0 + wm0 * kPad, s1, g, t4);
-            __syncthreads();
-        }
+        grid_wait();
+        dmma::stage_tile<NB, NB, true, kApplyThreads>(s2, inv, NB, 0, NB, 0, NB, tid);
+        __syncthreads();  // s1 is read no more
 #pragma unroll
         for (int j = 0; j < NT; ++j)
 #pragma unroll
@@ -502,6 +512,7 @@ __global__ void __launch_bounds__(kApplyThreads, 2) panel_apply_kernel(uint32_t 
                     bk[1] = v1;
                 acc[0][j][2 * h] = acc[0][j][2 * h + 1] = 0.0;
             }
+        dmma::cp_async_wait_all();
         __syncthreads();
         mma_k64<1, NT>(acc, s2 + wm0 * kPad, s1, g, t4);
 #pragma unroll
