@@ -167,6 +167,11 @@ __device__ __forceinline__ void panel_group_sync() { asm volatile("bar.sync 1, 1
 // The high word of |v|: an order on magnitudes to 2^-20, compared on the integer pipe.
 __device__ __forceinline__ int mag_hi(double v) { return __double2hiint(v) & 0x7FFFFFFF; }
 
+// The step after which panel_apply_kernel may start: late, since its waiting CTAs hold SMs that the
+// bulk update beside this kernel would take, but early enough for its loads and first product (after
+// step 5: n = 1024 387 us, 4096 2990; after 7: 399, 3020; after the last: 400, 3034).
+constexpr int kTopTrigger = 5;
+
 // update: panel p - 1 exists.  backup: rows 0 .. 63 of the panel's backup.  inv: (2, 64, 64), L^-1
 // and U^-1 of this block (a partial block padded with identity).
 template <bool VEC>
@@ -308,6 +313,8 @@ __global__ void __launch_bounds__(kTopThreads, 1) top_factor_kernel(uint32_t n, 
             }
         }
         __syncthreads();  // step k's rows and columns are final, update k - 1 is complete
+        if (k == kTopTrigger)
+            grid_launch_next();  // panel_apply_kernel: its first product needs nothing of this block
         if (k == NB / 8 - 1)
             break;
         // Column j of the update: X's column block j for j <= k, T's for j > k; the rows below take all
@@ -370,7 +377,6 @@ __global__ void __launch_bounds__(kTopThreads, 1) top_factor_kernel(uint32_t n, 
         if (warp < 4)
             panel_group_sync();
     }
-    grid_launch_next();  // panel_apply_kernel: its first product needs nothing of this block
     // the range of a pivot that pivot_rcp takes, and the limit of a multiplier (both to the high word:
     // what lies within 2^-20 of a bound takes the pivoting path, which is always right)
     const bool bad = lo <= __double2hiint(kPivotLo) || hi >= __double2hiint(kPivotHi) ||
