@@ -209,7 +209,9 @@ __device__ __forceinline__ void segment_induction(const Segment<T>& s, T px, T p
 // instructions and 15 others, where one call per point took 90 others (per-point votes inside
 // branches, scalar loads of the point) and was bound by instruction issue.  Pairs that need more
 // than eight terms on any lane (5 % of the warps' pairs on a 4096-ring wing, 2 % have a near pair)
-// take the per-lane forms.
+// take the per-lane forms.  Inside the cut-off the velocity is 0, not the value: 0 . n is NaN for a
+// normal that is not finite (a degenerate ring's), as in the kernel that evaluates every ring's own
+// lines.
 template <int NQ>
 __device__ __forceinline__ void segment_normal_values(const Segment<double>& s, const double (*__restrict__ pn)[6],
                                                       double tol2, double (&v)[NQ])
@@ -248,16 +250,16 @@ __device__ __forceinline__ void segment_normal_values(const Segment<double>& s, 
                 const double rh = rsqrt(hs[q]);
                 mag = atan2(-(hs[q] * rh) * s.len, xs[q]) * rh;
             }
-            v[q] = cut[q] ? 0.0 : v[q] * mag;
+            v[q] *= cut[q] ? 0.0 : mag;
         }
     } else if (__any_sync(0xFFFFFFFFu, worst > hi32(1e-4))) {
 #pragma unroll
         for (int q = 0; q < NQ; ++q)
-            v[q] = cut[q] ? 0.0 : v[q] * (-s.len * r[q] * F::sum_tier<8>(w[q]));
+            v[q] *= cut[q] ? 0.0 : -s.len * r[q] * F::sum_tier<8>(w[q]);
     } else {
 #pragma unroll
         for (int q = 0; q < NQ; ++q)
-            v[q] = cut[q] ? 0.0 : v[q] * (-s.len * r[q] * F::sum_tier<4>(w[q]));
+            v[q] *= cut[q] ? 0.0 : -s.len * r[q] * F::sum_tier<4>(w[q]);
     }
 }
 

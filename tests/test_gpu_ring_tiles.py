@@ -87,3 +87,33 @@ def test_too_many_points_are_refused():
     z = torch.zeros((n, 3), dtype=torch.float64, device="cuda")
     with pytest.raises(ValueError):
         Mesh(len(pos), elements).induction_matrix3(1e-6, torch.as_tensor(pos, device="cuda"), z, z)
+
+
+@pytest.mark.parametrize("tol", [1e-6, 0.3, 1e3])  # no line, some and all of them below the cut-off
+def test_normals_that_are_not_finite(tol):
+    """A NaN or infinite normal (a degenerate ring's) makes its row's entries NaN or infinite also where
+    every line of a ring is inside the cut-off: the same entries as in the per-ring kernel."""
+    import torch
+
+    from pyvl_b200 import _lib
+    from pyvl_b200.cvl import Mesh
+    from pyvl_b200.device import Workspace, ptr, stream_ptr
+
+    pos, elements = _fan(40, 4)
+    mesh = Mesh(len(pos), elements)
+    cps, nrm = _points(pos, 24, 3)
+    nrm[1], nrm[6, 2], nrm[11, 0] = np.nan, np.nan, np.inf
+    dev = [torch.as_tensor(a, device="cuda") for a in (pos, cps, nrm)]
+    got = mesh.induction_matrix3(tol, *dev).cpu().numpy()
+    d = mesh.device_arrays()
+    want = torch.zeros(got.shape, dtype=torch.float64, device="cuda")
+    ws, nb = Workspace.get(_lib.query("pvl_segments_workspace", mesh.n_lines, _lib.PVL_F64))
+    _lib.call("pvl_induction_normal", _lib.PVL_F64, mesh.n_points, mesh.n_lines, ptr(d["lines"]), ptr(dev[0]),
+              mesh.n_surfaces, ptr(d["offsets"]), ptr(d["surface_lines"]), len(cps), ptr(dev[1]), ptr(dev[2]), tol,
+              ptr(want), mesh.n_surfaces, ws, nb, stream_ptr())
+    want = want.cpu().numpy()
+    assert np.isnan(want[[1, 6]]).all()
+    assert np.array_equal(np.isfinite(got), np.isfinite(want))
+    ok = np.isfinite(want)
+    # as in the test above; 1e-12 of the largest finite entry
+    assert np.abs(got[ok] - want[ok]).max() <= 1e-12 * np.abs(want[ok]).max()
