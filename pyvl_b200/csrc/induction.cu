@@ -825,9 +825,14 @@ extern "C" int pvl_induction_normal(int precision, uint32_t n_points, uint32_t n
 namespace {
 
 // Threads of a ring-tile CTA: the candidate with the fewest idle lane-slots in the line loop
-// (rounds x threads - lines), ties to fewer threads.
-int ring_tile_threads(uint32_t max_tile_lines)
+// (rounds x threads - lines), ties to fewer threads.  Where the tile's values leave room for one CTA
+// per SM only, the most, since nothing else hides its latency: 1024 rings of 16 sides x 2048 points
+// with shared edges (1921 lines a tile) 533 us with 128 threads, 390 with 256 (a thread per ring that
+// evaluates its own lines: 460); 25 sides without (3200 lines) 729 and 498 (775).
+int ring_tile_threads(uint32_t max_tile_lines, size_t smem)
 {
+    if (smem > 112 * 1024)  // of 227 KB, 1 KB a CTA reserved
+        return 256;
     int best = kRingTile;
     uint64_t best_slots = ~0ull;
     for (int t : {128, 160, 192, 256}) {
@@ -885,7 +890,7 @@ extern "C" int pvl_induction_normal_tiled(uint32_t n_points, uint32_t n_lines, c
     auto* seg = static_cast<Segment<double>*>(ws);
     if (int r = prep_segments<double>(n_points, n_lines, lines, positions, nullptr, tol, seg, st))
         return r;
-    switch (ring_tile_threads(max_tile_lines)) {
+    switch (ring_tile_threads(max_tile_lines, smem)) {
     case 160:
         return launch_ring_tile<160>(grid, smem, st, n_surfaces, offsets, surface_lines, sl_local, tile_offsets,
                                      tile_lines, max_tile_lines, n_lines, seg, n_cp, cps, normals, tol, out, ld);

@@ -373,7 +373,9 @@ class Mesh:
         return d
 
     RING_TILE = 128  # rings per tile of pvl_induction_normal_tiled
-    TILE_LINES_MAX = 3200  # lines of a tile whose values at 8 control points fit its shared memory
+    # lines of a tile whose values at 8 control points fit its shared memory; up to there the tiled
+    # form is the faster one (1024 rings x 2048 points, 3200 lines a tile: 498 us against 775)
+    TILE_LINES_MAX = 3200
 
     def ring_tiles(self):
         """Per tile of RING_TILE consecutive rings: its distinct lines, and for every CSR entry

@@ -117,3 +117,10 @@ def test_normals_that_are_not_finite(tol):
     ok = np.isfinite(want)
     # as in the test above; 1e-12 of the largest finite entry
     assert np.abs(got[ok] - want[ok]).max() <= 1e-12 * np.abs(want[ok]).max()
+
+
+@pytest.mark.parametrize("sides,n_rings,n_cp", [(14, 128, 9), (15, 129, 8), (16, 130, 9), (25, 200, 17)])
+def test_tiles_that_fill_half_the_shared_memory(sides, n_rings, n_cp):
+    """Tiles of 1665 to 3073 lines: up to 1791 two CTAs share an SM, above one has it alone and takes more
+    threads."""
+    test_tiled_matrix_matches_per_ring_kernel(sides, n_rings, n_cp, True)
