@@ -381,15 +381,14 @@ size_t pivot_smem(uint32_t rows)
 constexpr int kTrsmCols = 128;
 
 template <typename T>
-__global__ void __launch_bounds__(kTrsmCols, 1) trsm_kernel(uint32_t n, uint32_t k0, uint32_t nb,
-                                                            T* __restrict__ A, uint32_t lda,
-                                                            const int32_t* __restrict__ ok, uint32_t panel,
-                                                            const int32_t* __restrict__ ipiv, int fast_u12)
+__global__ void __launch_bounds__(kTrsmCols, 1) trsm_kernel(uint32_t n, uint32_t k0, uint32_t nb, T* A,
+                                                            uint32_t lda, const int32_t* ok, uint32_t panel,
+                                                            const int32_t* ipiv, int fast_u12)
 {
     if (fast_u12) {
         pvl::panel::grid_launch_next();  // the next panel's top_factor_kernel waits for this one's end
         pvl::panel::grid_wait();         // panel_pivot_kernel's
-        if (ok[panel])
+        if (*static_cast<const volatile int32_t*>(ok + panel))
             return;  // the FP64 path formed U12 = L11^-1 A12 already and nothing was interchanged
     }
     extern __shared__ double tsm_raw[];
@@ -720,7 +719,8 @@ extern "C" int pvl_lu_factor(uint32_t n, double* A, uint32_t lda, int32_t* ipiv,
     init_perm_kernel<<<blocks_for(n, 256), 256, 0, st>>>(n, perm);
     PVL_LAUNCH_CHECK();
     const uint32_t n_panels = (n + NB - 1) / NB;
-    PVL_CUDA_CHECK(cudaMemsetAsync(w.reject, 0, sizeof(int32_t) * (n_panels + 1), st));
+    // reject, and ok behind it: no panel counts as accepted before its own check
+    PVL_CUDA_CHECK(cudaMemsetAsync(w.reject, 0, (size_t)((char*)w.tmp - (char*)w.reject), st));
     // Look-ahead: panel p's trailing update beyond panel p + 1 runs on the side stream, on all but
     // a share of the SMs, while panel p + 1's diagonal block, multipliers and row block (which
     // apply panel p's update to their own entries) run on `st`.  Panel p + 1's pivoting fallback,

@@ -73,9 +73,8 @@ __device__ __forceinline__ void mma_k64(double (&acc)[MT][NT][4], const double* 
 // acc = -C over the warp's 16 MT x 8 NT entries (rows from `row`, columns from `col`, valid below
 // m_end / n_end); entries outside are 0.
 template <int MT, int NT, bool VEC>
-__device__ __forceinline__ void load_neg(double (&acc)[MT][NT][4], const double* __restrict__ C, uint32_t ldc,
-                                         uint32_t row, uint32_t col, uint32_t m_end, uint32_t n_end, uint32_t g,
-                                         uint32_t t)
+__device__ __forceinline__ void load_neg(double (&acc)[MT][NT][4], const double* C, uint32_t ldc, uint32_t row,
+                                         uint32_t col, uint32_t m_end, uint32_t n_end, uint32_t g, uint32_t t)
 {
 #pragma unroll
     for (int i = 0; i < MT; ++i)
@@ -159,6 +158,9 @@ __device__ __forceinline__ void tiles(double* m, const int (&dst)[N], const int 
 // Programmatic dependent launch (the chain's kernels may be started before the one ahead of them in
 // the stream has ended): wait until it has, its writes visible; and let the next kernel start.
 // Every kernel launched so waits before it ends, so its own end implies all earlier ones'.
+// No parameter of a kernel that waits so is __restrict__: the kernel ahead still writes through the
+// same addresses when this one has started, and the qualifier would let the compiler read them
+// through the non-coherent path or ahead of the wait.
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_launch_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
@@ -176,11 +178,8 @@ constexpr int kTopTrigger = 5;
 // and U^-1 of this block (a partial block padded with identity).
 template <bool VEC>
 __global__ void __launch_bounds__(kTopThreads, 1) top_factor_kernel(uint32_t n, uint32_t k0, uint32_t nb, int update,
-                                                                    double* __restrict__ A, uint32_t lda,
-                                                                    double* __restrict__ backup,
-                                                                    double* __restrict__ inv,
-                                                                    int32_t* __restrict__ ipiv,
-                                                                    int32_t* __restrict__ reject)
+                                                                    double* A, uint32_t lda, double* backup,
+                                                                    double* inv, int32_t* ipiv, int32_t* reject)
 {
     extern __shared__ __align__(16) double top_smem[];
     TopSmem& s = *reinterpret_cast<TopSmem*>(top_smem);
@@ -423,11 +422,9 @@ constexpr size_t kApplySmem = (size_t)3 * NB * kPad * sizeof(double);
 
 template <bool VEC>
 __global__ void __launch_bounds__(kApplyThreads, 2) panel_apply_kernel(uint32_t n, uint32_t k0, int update,
-                                                                       double* __restrict__ A, uint32_t lda,
-                                                                       const double* __restrict__ inv,
-                                                                       double* __restrict__ backup,
-                                                                       double* __restrict__ backup_row,
-                                                                       int32_t* __restrict__ reject, uint32_t n_ltiles)
+                                                                       double* A, uint32_t lda, const double* inv,
+                                                                       double* backup, double* backup_row, int32_t* reject,
+                                                                       uint32_t n_ltiles)
 {
     constexpr int R = kApplyRows;
     extern __shared__ __align__(16) double apply_smem[];

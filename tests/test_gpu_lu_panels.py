@@ -87,3 +87,25 @@ def test_solution_with_the_bits_of_the_not_ready_mark():
     torch.cuda.synchronize()
     assert int(err.item()) == 0
     assert bool(torch.isnan(x).any())
+
+
+def test_workspace_of_an_accepted_factorisation_reused_for_a_rejected_one():
+    """The panels of the second matrix interchange rows where the first one's did not: their swaps and row
+    blocks are formed although the workspace remembers accepted panels."""
+    import torch
+
+    from pyvl_b200 import _lib
+    from pyvl_b200.device import ptr, stream_ptr
+
+    n = 640
+    ipiv = torch.zeros(2 * n, dtype=torch.int32, device="cuda")
+    info = torch.zeros(1, dtype=torch.int32, device="cuda")
+    nb = int(_lib.query("pvl_lu_workspace", n))
+    ws = torch.zeros(nb, dtype=torch.uint8, device="cuda")
+    for swapped in ((), (0, 3, 4, 9), (), tuple(range(10))):
+        A, _ = _system(n, swapped, 5)
+        M = torch.as_tensor(A, device="cuda")
+        _lib.call("pvl_lu_factor", n, ptr(M), n, ptr(ipiv), ptr(info), ptr(ws), nb, stream_ptr())
+        lu, piv = la.lu_factor(A)
+        assert np.array_equal(ipiv[:n].cpu().numpy(), piv)
+        assert rel(M.cpu().numpy(), lu) <= 1e-13
