@@ -7,6 +7,7 @@ from __future__ import annotations
 
 import ctypes
 import gc
+import threading
 
 import numpy as np
 import torch
@@ -60,29 +61,47 @@ def to_device_u32(a, device=None) -> torch.Tensor:
     return torch.from_numpy(arr.copy()).to(dev)
 
 
+class _CollectorHeld:
+    """The cyclic collector off, for all threads, from the first one's entry to the last one's exit;
+    then as it was."""
+
+    _lock = threading.Lock()
+    _inside = 0
+    _was_on = False
+
+    def __enter__(self):
+        cls = _CollectorHeld
+        with cls._lock:
+            if cls._inside == 0:
+                cls._was_on = gc.isenabled()
+                gc.disable()
+            cls._inside += 1
+
+    def __exit__(self, *exc):
+        cls = _CollectorHeld
+        with cls._lock:
+            cls._inside -= 1
+            if cls._inside == 0 and cls._was_on:
+                gc.enable()
+
+
 def capture_graph(fn) -> torch.cuda.CUDAGraph:
     """``fn`` (launches on fixed buffers, no host reads) captured as a CUDA graph.
 
     torch.cuda.graph without the device-wide synchronisation, garbage collection and emptied
     allocator cache of its entry (~1 ms a capture, more than a short run's steps take).  The
     cyclic collector is held off instead, so that nothing it frees reaches the CUDA runtime while
-    the stream captures."""
+    the stream captures (until the last of several threads' captures has ended)."""
     g = torch.cuda.CUDAGraph()
     cur = torch.cuda.current_stream()
     side = torch.cuda.Stream()
     side.wait_stream(cur)
-    collecting = gc.isenabled()
-    gc.disable()
-    try:
-        with torch.cuda.stream(side):
-            g.capture_begin()
-            try:
-                fn()
-            finally:
-                g.capture_end()
-    finally:
-        if collecting:
-            gc.enable()
+    with _CollectorHeld(), torch.cuda.stream(side):
+        g.capture_begin()
+        try:
+            fn()
+        finally:
+            g.capture_end()
     cur.wait_stream(side)
     return g
 
