@@ -607,6 +607,12 @@ int pvl_line_forces(uint32_t n_lines, const uint32_t* primal_lines, const uint32
                     const double* circ, const double* positions, const double* velocity,
                     double* out, void* stream);
 
+/* ------------------------------------------------------------------ streams */
+
+/* A new non-blocking stream of the current device in *stream, the caller's own (cudaStreamDestroy
+ * ends it): a graph capture needs one that nothing else enqueues on.  No reference counterpart. */
+int pvl_stream_create(void** stream);
+
 /* ------------------------------------------------------------------ measurement */
 
 /* Number of kernels this library has enqueued since it was loaded (all threads).  No

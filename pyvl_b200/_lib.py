@@ -125,6 +125,7 @@ SIGNATURES = {
     "pvl_mlp_adam": (_I, [_P, _P, _P, _P, _P, _U, ctypes.c_float, ctypes.c_float, ctypes.c_float, ctypes.c_float,
                           _P]),
     "pvl_mlp_to_bf16": (_I, [_P, _P, _P]),
+    "pvl_stream_create": (_I, [_P]),
     "pvl_launch_count": (ctypes.c_ulonglong, []),
 }
 

@@ -22,7 +22,7 @@ import torch
 
 from . import _lib
 from .cvl import Mesh
-from .device import ptr, require_cuda, stream_ptr, to_device_u32
+from .device import capture_graph, ptr, require_cuda, stream_ptr, to_device_u32
 from .engine import wake_node_columns, wake_ring_connectivity, wake_row0_mesh, wake_spec_from_te
 
 RING_JOB = np.dtype([("cp_begin", "<u4"), ("n_cp", "<u4"), ("ring_begin", "<u4"), ("n_rings", "<u4"),
@@ -515,11 +515,8 @@ class BatchEngine:
         if self.iteration == 0:
             raise RuntimeError("capture after the first step")
         torch.cuda.synchronize()
-        g = torch.cuda.CUDAGraph()
         n0 = _lib.lib().pvl_launch_count()
-        with torch.cuda.graph(g):
-            self._step_body(with_wake=True)
-        self.graph = g
+        self.graph = capture_graph(lambda: self._step_body(with_wake=True))
         self.graph_kernels = int(_lib.lib().pvl_launch_count() - n0)  # kernels each replay runs
 
     def failures(self) -> int:

@@ -12,6 +12,8 @@ import threading
 import numpy as np
 import torch
 
+from . import _lib
+
 
 def require_cuda() -> torch.device:
     """Return the current CUDA device or raise: the hot path has no CPU fallback."""
@@ -85,6 +87,33 @@ class _CollectorHeld:
                 gc.enable()
 
 
+class _CaptureStreams:
+    """Streams that only captures use, each by one capture at a time: as many per device as captures
+    have been under way at once.  (torch.cuda.Stream() hands out the same few dozen handles in turn,
+    so that its stream may be one on which another thread is enqueuing work, which would end up in
+    the graph.)"""
+
+    _lock = threading.Lock()
+    _free: dict = {}
+
+    def __init__(self, device: int):
+        self.device = device
+
+    def __enter__(self):
+        with self._lock:
+            free = self._free.setdefault(self.device, [])
+            self.stream = free.pop() if free else None
+        if self.stream is None:
+            handle = ctypes.c_void_p()
+            _lib.call("pvl_stream_create", ctypes.byref(handle))
+            self.stream = torch.cuda.ExternalStream(handle.value, device=self.device)
+        return self.stream
+
+    def __exit__(self, *exc):
+        with self._lock:
+            self._free[self.device].append(self.stream)
+
+
 def capture_graph(fn) -> torch.cuda.CUDAGraph:
     """``fn`` (launches on fixed buffers, no host reads) captured as a CUDA graph.
 
@@ -94,15 +123,15 @@ def capture_graph(fn) -> torch.cuda.CUDAGraph:
     the stream captures (until the last of several threads' captures has ended)."""
     g = torch.cuda.CUDAGraph()
     cur = torch.cuda.current_stream()
-    side = torch.cuda.Stream()
-    side.wait_stream(cur)
-    with _CollectorHeld(), torch.cuda.stream(side):
-        g.capture_begin()
-        try:
-            fn()
-        finally:
-            g.capture_end()
-    cur.wait_stream(side)
+    with _CaptureStreams(require_cuda().index) as side:
+        side.wait_stream(cur)
+        with _CollectorHeld(), torch.cuda.stream(side):
+            g.capture_begin()
+            try:
+                fn()
+            finally:
+                g.capture_end()
+        cur.wait_stream(side)
     return g
 
 

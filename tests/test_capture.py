@@ -4,6 +4,7 @@ and the streams replaced by stand-ins.  No GPU needed."""
 import contextlib
 import gc
 import threading
+from pathlib import Path
 
 import pytest
 
@@ -11,7 +12,8 @@ from pyvl_b200 import device
 
 
 class _Stream:
-    cuda_stream = 0
+    def __init__(self, handle=0, device=None):
+        self.handle = handle
 
     def wait_stream(self, other):
         pass
@@ -27,12 +29,27 @@ class _Graph:
 
 @pytest.fixture
 def stand_ins(monkeypatch):
+    entered, made = [], []
+
+    def create(name, out):
+        assert name == "pvl_stream_create"
+        made.append(len(made) + 1)
+        out._obj.value = made[-1]
+
+    @contextlib.contextmanager
+    def enter(s):
+        entered.append(s.handle)
+        yield
+
+    monkeypatch.setattr(device._lib, "call", create)
+    monkeypatch.setattr(device, "require_cuda", lambda: device.torch.device("cuda", 0))
+    monkeypatch.setattr(device._CaptureStreams, "_free", {})
     monkeypatch.setattr(device.torch.cuda, "CUDAGraph", _Graph)
-    monkeypatch.setattr(device.torch.cuda, "Stream", _Stream)
+    monkeypatch.setattr(device.torch.cuda, "ExternalStream", _Stream)
     monkeypatch.setattr(device.torch.cuda, "current_stream", lambda *a: _Stream())
-    monkeypatch.setattr(device.torch.cuda, "stream", lambda s: contextlib.nullcontext())
+    monkeypatch.setattr(device.torch.cuda, "stream", enter)
     on = gc.isenabled()
-    yield
+    yield entered
     (gc.enable if on else gc.disable)()
 
 
@@ -81,3 +98,21 @@ def test_collector_is_back_after_a_capture_that_fails(stand_ins):
     with pytest.raises(RuntimeError, match="in the capture"):
         device.capture_graph(fails)
     assert gc.isenabled()
+
+
+def test_a_capture_has_its_stream_to_itself(stand_ins):
+    """One after the other, also after one that failed: the same stream.  One inside the other: another."""
+    def fails():
+        raise RuntimeError("in the capture")
+
+    device.capture_graph(lambda: None)
+    with pytest.raises(RuntimeError):
+        device.capture_graph(fails)
+    device.capture_graph(lambda: device.capture_graph(lambda: None))
+    device.capture_graph(lambda: None)
+    assert stand_ins[:4] == [1, 1, 1, 2] and stand_ins[4] in (1, 2)
+
+
+def test_captures_take_one_route():
+    sources = sorted((Path(device.__file__).parent).rglob("*.py"))
+    assert sources and not [p.name for p in sources if "cuda.graph(" in p.read_text()]

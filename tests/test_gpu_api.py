@@ -199,3 +199,26 @@ def test_postprocess_fields_match_oracle():
         rho = settings.flow_conditions.get_density(t, cps)
         p = -rho * np.vecdot(ind, 0.5 * ind + np.broadcast_to(case.freestream, cps.shape), axis=-1)
         assert rel(pres[i], p) <= PARITY, i
+
+
+def test_capture_stream_is_no_stream_of_the_pool():
+    """torch.cuda.Stream() hands out a fixed set of streams in turn; a capture must not run on one of them,
+    on which another thread may be enqueuing work."""
+    import torch
+
+    from pyvl_b200.device import capture_graph
+
+    pool = {torch.cuda.Stream().cuda_stream for _ in range(64)}
+    x = torch.zeros(4, device="cuda")
+    used = []
+
+    def work():
+        used.append(torch.cuda.current_stream().cuda_stream)
+        x.add_(1.0)
+
+    graphs = [capture_graph(work) for _ in range(3)]
+    assert len(set(used)) == 1 and used[0] not in pool
+    for g in graphs:
+        g.replay()
+    torch.cuda.synchronize()
+    assert x.tolist() == [3.0] * 4
