@@ -211,7 +211,8 @@ __global__ void __launch_bounds__(kTopThreads, 1) top_factor_kernel(uint32_t n, 
             for (int h = 0; h < 2; ++h) {
                 const uint32_t r = wm0 + g + 16 * i + 8 * h, c = wn0 + 2 * t4 + 8 * j;
                 const double2 v = make_double2(-acc[i][j][2 * h], -acc[i][j][2 * h + 1]);
-                *reinterpret_cast<double2*>(backup + r * NB + c) = v;  // past nb: never read
+                if (r < nb)  // the backup has n rows
+                    *reinterpret_cast<double2*>(backup + r * NB + c) = v;  // columns past nb: never read
                 *reinterpret_cast<double2*>(&s.xt[r][NB + c]) = v;
                 const double2 e = make_double2(r == c ? 1.0 : 0.0, r == c + 1 ? 1.0 : 0.0);
                 *reinterpret_cast<double2*>(&s.xt[r][c]) = e;

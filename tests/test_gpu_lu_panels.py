@@ -109,3 +109,24 @@ def test_workspace_of_an_accepted_factorisation_reused_for_a_rejected_one():
         lu, piv = la.lu_factor(A)
         assert np.array_equal(ipiv[:n].cpu().numpy(), piv)
         assert rel(M.cpu().numpy(), lu) <= 1e-13
+
+
+@pytest.mark.parametrize("n", [1, 2, 31, 63, 65])
+def test_backup_stays_inside_its_rows(n):
+    """A panel's backup has n rows of 64 values at the head of the workspace; the region behind it, the FP32
+    factorisation's top block, is not the FP64 one's to write."""
+    import torch
+
+    from pyvl_b200 import _lib
+    from pyvl_b200.device import ptr, stream_ptr
+
+    A, b = _system(n, (), n)
+    M = torch.as_tensor(A, device="cuda")
+    ipiv = torch.zeros(2 * n, dtype=torch.int32, device="cuda")
+    info = torch.zeros(1, dtype=torch.int32, device="cuda")
+    nb = int(_lib.query("pvl_lu_workspace", n))
+    ws = torch.full((nb,), 255, dtype=torch.uint8, device="cuda")
+    _lib.call("pvl_lu_factor", n, ptr(M), n, ptr(ipiv), ptr(info), ptr(ws), nb, stream_ptr())
+    begin = -(-n * 64 * 8 // 256) * 256
+    assert bool((ws[begin:begin + 64 * 64 * 8] == 255).all())
+    assert rel(M.cpu().numpy(), la.lu_factor(A)[0]) <= 1e-13
