@@ -332,7 +332,9 @@ int pvl_wake_shed(uint32_t n_shed, uint32_t line_rows, const double* old_circ,
 
 /* ------------------------------------------------------------------ dense solve */
 
-/* Scratch for pvl_lu_factor / pvl_lu_solve. */
+/* Scratch for pvl_lu_factor / pvl_lu_solve (one buffer for both: the factorisation leaves the
+ * inverted diagonal blocks in it).  About 2 KB per row; for odd n an n x n copy of the matrix on
+ * top (rows of 128-byte multiples: 211 MB at n = 5121), in which it is factored. */
 size_t pvl_lu_workspace(uint32_t n);
 size_t pvl_lu_solve_workspace(uint32_t n);
 
@@ -461,7 +463,7 @@ int pvl_pad_convert_f32(uint32_t n, const double* a, uint32_t lda, float* b, uin
  * factorisation of the mixed path: the FP64 factorisation's panel/pivot/TRSM steps in FP32
  * and the trailing update on the tensor cores (pvl_gemm_tf32).  ipiv as pvl_lu_factor
  * (2n int32: LAPACK interchanges, then the row permutation).  lda a multiple of 4 and A
- * 16-byte aligned; ws of pvl_lu32_workspace(n) bytes, which keeps the inverted diagonal
+ * 16-byte aligned; ws of pvl_lu32_workspace(n) bytes (about 2 KB per row), which keeps the inverted diagonal
  * blocks for pvl_lu32_inverse.  *err = 1 if a tensor-core wait timed out.  Replaces
  * scipy.linalg.lu_factor (solver.py:223) inside the preconditioner only. */
 size_t pvl_lu32_workspace(uint32_t n);

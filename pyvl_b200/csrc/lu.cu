@@ -53,13 +53,15 @@ struct LuWs {
 // Row stride of LuWs::even, 0 where the matrix is factored in place.
 uint32_t even_stride(uint32_t n) { return n % 2 ? (n + 15) & ~15u : 0; }
 
-size_t lu_ws_bytes(uint32_t n)
+// lu32: the FP32 factorisation's, which has no copy of the matrix.
+size_t lu_ws_bytes(uint32_t n, bool lu32 = false)
 {
     return align256((size_t)n * NB * sizeof(double)) + align256((size_t)NB * NB * sizeof(double)) +
            align256(((size_t)n / NB + 2) * sizeof(int32_t)) +
            align256(((size_t)n / NB + 2) * sizeof(int32_t)) +
            align256((size_t)n * sizeof(double)) + align256(((size_t)n + kRB - 1) / kRB * 2 * kRB * kRB * sizeof(double)) +
-           align256((size_t)NB * n * sizeof(double)) + align256((size_t)n * even_stride(n) * sizeof(double));
+           align256((size_t)NB * n * sizeof(double)) +
+           (lu32 ? 0 : align256((size_t)n * even_stride(n) * sizeof(double)));
 }
 
 LuWs carve(void* ws, uint32_t n)
@@ -963,7 +965,7 @@ int rank64_update(uint32_t M, uint32_t cols, const float* A, uint32_t lda, const
 }
 }  // namespace
 
-extern "C" size_t pvl_lu32_workspace(uint32_t n) { return lu_ws_bytes(n); }
+extern "C" size_t pvl_lu32_workspace(uint32_t n) { return lu_ws_bytes(n, true); }
 
 extern "C" int pvl_lu32_factor(uint32_t n, float* A, uint32_t lda, int32_t* ipiv, int32_t* info, int32_t* err,
                                void* ws, size_t ws_bytes, void* stream)
@@ -974,8 +976,8 @@ extern "C" int pvl_lu32_factor(uint32_t n, float* A, uint32_t lda, int32_t* ipiv
         return pvl_fail(PVL_ERR_ARG, "pvl_lu32_factor: null pointer argument");
     if (lda < n || lda % 4 || ((uintptr_t)A & 15u))
         return pvl_fail(PVL_ERR_ARG, "pvl_lu32_factor: lda must be >= n and a multiple of 4, A 16-byte aligned");
-    if (ws_bytes < lu_ws_bytes(n))
-        return pvl_fail(PVL_ERR_ALLOC, "pvl_lu32_factor: workspace %zu < %zu", ws_bytes, lu_ws_bytes(n));
+    if (ws_bytes < lu_ws_bytes(n, true))
+        return pvl_fail(PVL_ERR_ALLOC, "pvl_lu32_factor: workspace %zu < %zu", ws_bytes, lu_ws_bytes(n, true));
     cudaStream_t st = (cudaStream_t)stream;
     LuWs w = carve(ws, n);
     float* backup = reinterpret_cast<float*>(w.backup);
@@ -1034,7 +1036,7 @@ extern "C" int pvl_lu32_inverse(uint32_t n, const float* LU, uint32_t lda, const
         (((uintptr_t)LU | (uintptr_t)X | (uintptr_t)Y) & 15u))
         return pvl_fail(PVL_ERR_ARG, "pvl_lu32_inverse: leading dimensions must be >= n and multiples of 4, "
                                      "arrays 16-byte aligned");
-    if (ws_bytes < lu_ws_bytes(n))
+    if (ws_bytes < lu_ws_bytes(n, true))
         return pvl_fail(PVL_ERR_ALLOC, "pvl_lu32_inverse: workspace too small");
     cudaStream_t st = (cudaStream_t)stream;
     LuWs w = carve(ws, n);

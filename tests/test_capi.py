@@ -185,3 +185,11 @@ def test_argument_errors_are_reported_before_any_device_work():
         create(v32=fake + 4)
     with pytest.raises(_lib.PvlError, match="workspace"):
         create(ws_bytes=args["ws_bytes"] - 1)
+
+
+@pytest.mark.parametrize("n", [1, 63, 451, 5121, 16385])
+def test_fp32_lu_workspace_has_no_copy_of_the_matrix(n):
+    """Only the FP64 factorisation of an odd order works in a copy; the FP32 one's scratch grows by the row."""
+    below, above = (int(_lib.query("pvl_lu32_workspace", n + d)) for d in (-1, 1))
+    assert below <= int(_lib.query("pvl_lu32_workspace", n)) <= above
+    assert int(_lib.query("pvl_lu_workspace", n)) >= int(_lib.query("pvl_lu32_workspace", n)) + 8 * n * n
