@@ -130,3 +130,42 @@ def test_backup_stays_inside_its_rows(n):
     begin = -(-n * 64 * 8 // 256) * 256
     assert bool((ws[begin:begin + 64 * 64 * 8] == 255).all())
     assert rel(M.cpu().numpy(), la.lu_factor(A)[0]) <= 1e-13
+
+
+@pytest.mark.parametrize("n,pad,swapped", [
+    (130, 3, ()), (130, 1, (2,)), (706, 1, ()), (706, 1, (0, 11)), (2110, 1, ()), (2110, 3, (31, 32)),
+])
+def test_odd_row_strides_with_ragged_last_panels(n, pad, swapped):
+    """An even order with an odd row stride is factored in place with 8-byte copies: partial last panels
+    after an update, and trailing tiles that are not full."""
+    test_lu_and_solve_match_lapack(n, pad, swapped)
+
+
+@pytest.mark.parametrize("n,lda,swapped", [(64, 64, ()), (130, 132, (2,)), (706, 706, ()), (706, 708, (0, 11))])
+def test_matrix_that_is_not_16_byte_aligned(n, lda, swapped):
+    """An even order and row stride, but a base 8 bytes off a 16-byte boundary."""
+    import torch
+
+    from pyvl_b200 import _lib
+    from pyvl_b200.device import ptr, stream_ptr
+
+    A, b = _system(n, swapped, n + lda)
+    store = torch.full((n * lda + 1,), float("nan"), dtype=torch.float64, device="cuda")
+    M = store[1:].view(n, lda)
+    assert M.data_ptr() % 16 == 8
+    M[:, :n] = torch.as_tensor(A)
+    ipiv = torch.zeros(2 * n, dtype=torch.int32, device="cuda")
+    info = torch.zeros(1, dtype=torch.int32, device="cuda")
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    nb = int(_lib.query("pvl_lu_workspace", n))
+    ws = torch.full((nb,), 255, dtype=torch.uint8, device="cuda")
+    x = torch.as_tensor(b, device="cuda")
+    _lib.call("pvl_lu_factor", n, ptr(M), lda, ptr(ipiv), ptr(info), ptr(ws), nb, stream_ptr())
+    _lib.call("pvl_lu_solve", n, ptr(M), lda, ptr(ipiv), ptr(x), ptr(err), ptr(ws), nb, stream_ptr())
+    torch.cuda.synchronize()
+    assert int(info.item()) == 0 and int(err.item()) == 0
+    lu, piv = la.lu_factor(A)
+    assert np.array_equal(ipiv[:n].cpu().numpy(), piv)
+    assert rel(M[:, :n].cpu().numpy(), lu) <= 1e-13
+    assert bool(torch.isnan(M[:, n:]).all()) and bool(torch.isnan(store[:1]).all())
+    assert rel(x.cpu().numpy(), la.lu_solve((lu, piv), b)) <= 1e-12
