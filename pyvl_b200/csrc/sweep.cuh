@@ -10,7 +10,7 @@
 // |p - o| + |r1 - o| instead of |p - r1|; the points of one CTA are neighbours (ring or
 // wake-node order, or one case of a batch), so |p - o| stays of the order of the body.
 // Everything after c and t1 -- h^2, x = h^2 + t1 t2, the far-field series with the Newton
-// reciprocal, the atan2 form for near pairs, the cut-off -- is segment_induction<double, true>,
+// reciprocal, the atan2 form for near pairs, the cut-off -- is segment_induction's, scaled by gamma,
 // with w = h^2 len^2 / x^2 formed as h^2 (len / x)^2.
 #pragma once
 
