@@ -491,15 +491,14 @@ __global__ void __launch_bounds__(pvl::dmma::kUpdThreads, 1) dmma_update_kernel(
                                  r.b_row, t0, t1);
 }
 
-// CTAs (one per SM) of the update of an m x m block: the rest of the SMs is left to the next
-// panel's kernels, whose share of the work grows as the block shrinks (a share of 256, 400 or 600
-// columns' worth: n = 3072 1776, 1786, 1796 us; n = 4096 3127, 3136, 3163; 128: 70 us more).
-constexpr uint32_t kBulkShare = 256;
-uint32_t bulk_ctas(int sms, uint32_t m)
-{
-    const uint32_t free_sms = 8 + (uint32_t)sms * kBulkShare / (m + 4 * kBulkShare);
-    return (uint32_t)std::max(1, sms - (int)free_sms);
-}
+// SMs that a trailing update (one CTA per SM) leaves to the next panel's kernels meanwhile: one for the
+// diagonal block, and one for the first CTAs of the multipliers' kernel, which is started while that
+// block is still being factored; the others follow as the update's CTAs end.  A share that grows as the block
+// shrinks (8 and 256 columns' worth of the SMs, from before the chain's kernels were launched as
+// dependents) no longer pays at any size: n = 2048 838 us with it, 827, 819, 821, 819 with 8, 4, 2 and
+// 1 SMs; 3072 1646, 1619, 1608, 1599, 1598; 4096 2983, 2927, 2907, 2894, 2892; 8192 16956, 16615,
+// 16536, 16506, 16500; up to 1536 all alike.
+constexpr int kChainSms = 2;
 
 // A kernel of the chain, allowed to start before the kernel ahead of it in the stream has ended
 // (lu_panel.cuh grid_wait): its launch, and what it needs of older kernels only, run beside that
@@ -771,7 +770,7 @@ extern "C" int pvl_lu_factor(uint32_t n, double* A, uint32_t lda, int32_t* ipiv,
         if (below <= NB)
             continue;  // the next panel is the last: it applies this update itself
         const uint32_t rest = k0 + 2 * NB;
-        const UpdRect r = upd_rect(rest, rest, n - rest, n - rest, k0, bulk_ctas(sms, n - rest));
+        const UpdRect r = upd_rect(rest, rest, n - rest, n - rest, k0, (uint32_t)std::max(1, sms - kChainSms));
         PVL_CUDA_CHECK(cudaEventRecord(side->fork, st));
         PVL_CUDA_CHECK(cudaStreamWaitEvent(side->s, side->fork, 0));
         void* uargs[] = {(void*)&A, (void*)&lda, (void*)&r};
