@@ -120,7 +120,19 @@ def capture_graph(fn) -> torch.cuda.CUDAGraph:
     torch.cuda.graph without the device-wide synchronisation, garbage collection and emptied
     allocator cache of its entry (~1 ms a capture, more than a short run's steps take).  The
     cyclic collector is held off instead, so that nothing it frees reaches the CUDA runtime while
-    the stream captures (until the last of several threads' captures has ended)."""
+    the stream captures (until the last of several threads' captures has ended).  The allocator
+    gives no cached block back while a stream captures, so a capture that finds the memory full is
+    repeated after the collection and with the cache emptied."""
+    try:
+        return _capture(fn)
+    except torch.OutOfMemoryError:
+        pass  # the failed capture's tensors go with the exception
+    gc.collect()
+    torch.cuda.empty_cache()
+    return _capture(fn)
+
+
+def _capture(fn) -> torch.cuda.CUDAGraph:
     g = torch.cuda.CUDAGraph()
     cur = torch.cuda.current_stream()
     with _CaptureStreams(require_cuda().index) as side:

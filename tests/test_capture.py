@@ -116,3 +116,24 @@ def test_a_capture_has_its_stream_to_itself(stand_ins):
 def test_captures_take_one_route():
     sources = sorted((Path(device.__file__).parent).rglob("*.py"))
     assert sources and not [p.name for p in sources if "cuda.graph(" in p.read_text()]
+
+
+def test_a_capture_that_finds_the_memory_full_is_repeated(stand_ins, monkeypatch):
+    import torch
+
+    emptied, tries = [], []
+    monkeypatch.setattr(torch.cuda, "empty_cache", lambda: emptied.append(len(tries)))
+
+    def full_once():
+        tries.append(gc.isenabled())
+        if len(tries) == 1:
+            raise torch.OutOfMemoryError("full")
+
+    device.capture_graph(full_once)
+    assert emptied == [1] and tries == [False, False]
+
+    def always_full():
+        raise torch.OutOfMemoryError("full")
+
+    with pytest.raises(torch.OutOfMemoryError):
+        device.capture_graph(always_full)

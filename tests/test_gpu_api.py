@@ -222,3 +222,25 @@ def test_capture_stream_is_no_stream_of_the_pool():
         g.replay()
     torch.cuda.synchronize()
     assert x.tolist() == [3.0] * 4
+
+
+def test_capture_with_the_memory_held_by_the_allocator_cache():
+    """A capture whose step allocates succeeds when only cached blocks stand in its way."""
+    import torch
+
+    from pyvl_b200.device import capture_graph
+
+    out = torch.zeros(1, device="cuda")
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    cached = torch.empty(512 << 20, dtype=torch.uint8, device="cuda")
+    del cached  # 512 MB stay in the cache
+    total = torch.cuda.get_device_properties(0).total_memory
+    torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (64 << 20)) / total)
+    try:
+        g = capture_graph(lambda: out.add_(torch.ones(64 << 20, device="cuda").sum()))  # 256 MB
+        g.replay()
+        torch.cuda.synchronize()
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    assert out.item() == float(64 << 20)
