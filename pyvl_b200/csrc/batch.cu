@@ -135,7 +135,7 @@ __global__ void __launch_bounds__(128) batched_ring_kernel(const RingJob* __rest
 // each thread sums its ring's signed entries (sl_local: each CSR entry's position in its
 // tile's list), in CSR order.  Adjacent rings share lines, so a quad mesh needs ~0.57 line
 // evaluations per (point, ring line) instead of one.  Lines and sums as in ring_tile_kernel
-// (induction.cu): 64 wings of 128 to 2048 rings, 716 -> 529 us.
+// (induction.cu): 64 wings of 128 to 2048 rings, 716 -> 526 us.
 // FOLD (implicit wake blocks): the block is not stored; the value of control point i and
 // first-row ring j (shedding line shed = J.ring_begin + j) is folded straight into the case's
 // system matrix, A[i, adj[2 shed + 1]] -= v and A[i, adj[2 shed]] += v (out_begin / ld = the

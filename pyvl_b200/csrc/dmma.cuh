@@ -60,10 +60,13 @@ __device__ __forceinline__ void cp_async_wait_all()
 // fetches, the other's MMAs keep the tensor pipe busy.  The A blocks stream into the group's
 // two-deep ring by cp.async, one tile ahead; C goes from global memory to registers while the
 // tile is multiplied (the product is formed by itself and subtracted at the end) and back, and the
-// next tile's C is prefetched into L2 meanwhile.  Against one group of eight warps per CTA with C in
-// the ring, n = 4096: 3323 -> 3243 us with two groups of four warps, 3167 with two of eight (four
-// warps per scheduler hide the fragment loads), 3140 with the prefetch.  4032 x 4032: 104 us, of
-// which the MMAs need 66 at their rate and C's traffic alone 69.
+// next tile's C is prefetched into L2 meanwhile.  What each part gave to the factorisation of 4096
+// (when the rest of it took 0.2 ms more than now): one group of eight warps per CTA with C in the ring
+// 3323 us, two groups of four warps 3243, two of eight 3167 (four warps per scheduler hide the
+// fragment loads), with the prefetch 3140.  The first update of n = 4096, 3968 x 3968: 96 us, the
+// FP64 tensor pipe active 66 % of it; a 4032 x 4032 one on 133 SMs took 106 us, 82 with C's traffic
+// left out and 69 with the MMAs left out (which need 66 at the pipe's rate): the two overlap only in
+// part.
 constexpr int kUpdTile = 64;
 constexpr int kUpdGroups = 2;  // (update_tiles names one barrier for each)
 constexpr int kUpdGroupThreads = 256;
@@ -154,7 +157,7 @@ __device__ __forceinline__ void update_tiles(UpdSmem& s, int group, uint32_t tid
         const uint32_t i0 = ti * kUpdTile, j0 = tj * kUpdTile;
         const uint32_t me = min((uint32_t)kUpdTile, m - i0), ne = min((uint32_t)kUpdTile, nn - j0);
         double* const cw = Cm + (size_t)(row0 + i0 + wm0 + g) * ld + col0 + j0 + wn0 + 2 * t4;
-        // C of this warp's 32 x 32: entry h of (i, j) is row wm0 + 16 i + 8 h + g
+        // C of this warp's 32 x 16 (32 x 8 NT): entry h of (i, j) is row wm0 + 16 i + 8 h + g
         double2 c[MT][NT][2];
 #pragma unroll
         for (int i = 0; i < MT; ++i)

@@ -122,12 +122,13 @@ __global__ void __launch_bounds__(kRingThreads) ring_matrix_kernel(
 // ~0.57 line evaluations per (point, ring line) instead of one.  The CTA has THREADS >=
 // kRingTile threads (chosen per launch from the largest tile's line count, so that the line
 // loop's last round is not mostly idle: 292 lines take two rounds of 160 threads instead of
-// three of 128); the first kRingTile of them sum the rings.  4096 x 4096: 239 -> 186 us with two
+// three of 128); the first kRingTile of them sum the rings.  4096 x 4096: 239 -> 185 us with two
 // points per thread between votes (segment_normal_values, 239 -> 227) and sums without tests
-// (RingEntries, 227 -> 186); bound by FP64 issue (40 instructions a pair, 29 M pairs of full warps).
+// (RingEntries, 227 -> 185).  Bound by instruction issue (active 67 % of the time), the FP64 pipe (51 %)
+// the busiest: 40 FP64 instructions of ~109 in all, ring sums included, for each of 38 M pairs.
 constexpr int kRingTile = 128;
-constexpr int kTileNQ = 2;    // points a thread works together (4096 rings and points: 1: 194 us, 2: 186, 4: 213)
-constexpr int kTileCPB = 8;   // control points per CTA (8: 186 us, 16: 185 us; 28.7 and 33.3 us for 1280 rings)
+constexpr int kTileNQ = 2;    // points a thread works together (4096 rings and points: 1: 193 us, 2: 185, 4: 211)
+constexpr int kTileCPB = 8;   // control points per CTA (8: 185 us, 16: 182 us; 28.7 and 32.9 us for 1280 rings)
 
 template <int THREADS>
 __global__ void __launch_bounds__(THREADS) ring_tile_kernel(uint32_t n_surfaces, const uint32_t* __restrict__ off,

@@ -41,7 +41,7 @@ inline unsigned blocks_for(size_t n, unsigned t) { return (unsigned)((n + t - 1)
 
 struct LuWs {
     double* backup;         // (n, NB) copy of the current panel before speculation
-    double* top_out;        // (NB, NB) speculative top block (FP32 path)
+    double* top_out;        // (NB, NB) speculative top block (FP32 path only)
     int32_t* reject;        // per panel: the speculation failed
     int32_t* ok;            // per panel: speculative factors accepted
     double* tmp;            // (n) vector of the blocked solve
@@ -502,7 +502,8 @@ constexpr int kChainSms = 2;
 
 // A kernel of the chain, allowed to start before the kernel ahead of it in the stream has ended
 // (lu_panel.cuh grid_wait): its launch, and what it needs of older kernels only, run beside that
-// one's end.  n = 451 223 -> 202 us, 1024 436 -> 394, 2048 937 -> 857, 4096 3106 -> 3016.
+// one's end.  As ordinary launches n = 451 227 us, 1024 447, 2048 974, 4096 3036, 5121 5357; so 200,
+// 387, 832, 2897, 5223.
 cudaError_t launch_chained(const void* fn, dim3 grid, unsigned threads, void** args, size_t smem, cudaStream_t st)
 {
     cudaLaunchAttribute at{};
@@ -691,9 +692,9 @@ extern "C" int pvl_lu_factor(uint32_t n, double* A, uint32_t lda, int32_t* ipiv,
     if (int rc = side_stream(dev, side))
         return rc;
     // 16-byte operand copies need even row strides: a matrix of odd order is factored in a copy with
-    // one (5121: 7.1 ms in place with 8-byte copies; 128-byte aligned rows; an
-    // odd last column is then copied with the padding after it).  An even order with an odd stride
-    // keeps the 8-byte copies.
+    // one and 128-byte aligned rows (5121: 7.0 ms in place with 8-byte copies, 5.2 so; 451: 213 and
+    // 200 us); an odd last column is then copied with the padding after it.  An even order with an odd
+    // stride keeps the 8-byte copies.
     const dim3 copy_grid(blocks_for(n, 256), std::min<uint32_t>(n, 1024));
     double* const given = A;
     const uint32_t given_lda = lda;

@@ -117,7 +117,7 @@ __device__ __forceinline__ void load_neg(double (&acc)[MT][NT][4], const double*
 // What bounds it is latency, not the operations: measured with clock stamps, ~3000 cycles until the
 // operands are there, 4300 for the corner's product on one SM, eight steps of ~2000 (the 8 x 8
 // block 950, the solves 200, the barrier 200, the next row and column blocks 600), 3500 for the
-// stores; 19 us a block against 37 us (plus a separate update launch) with one barrier per column.
+// stores; 19-21 us a block against 37 us (plus a separate update launch) with one barrier per column.
 constexpr int kTopPad = 132;  // row stride of xt in doubles (132 = 4 mod 16, as kPad)
 struct __align__(16) TopSmem {
     double xt[NB][kTopPad];  // X in columns 0 .. 63, T in columns 64 .. 127
@@ -171,7 +171,7 @@ __device__ __forceinline__ int mag_hi(double v) { return __double2hiint(v) & 0x7
 
 // The step after which panel_apply_kernel may start: late, since its waiting CTAs hold SMs that the
 // bulk update beside this kernel would take, but early enough for its loads and first product (after
-// step 5: n = 1024 387 us, 4096 2990; after 7: 399, 3020; after the last: 400, 3034).
+// steps 3, 4 or 5: n = 1024 387 us, 4096 2898; after 6: 392, 2916; after 7, the last: 397, 2923).
 constexpr int kTopTrigger = 5;
 
 // update: panel p - 1 exists.  backup: rows 0 .. 63 of the panel's backup.  inv: (2, 64, 64), L^-1
@@ -414,9 +414,9 @@ __global__ void __launch_bounds__(kTopThreads, 1) top_factor_kernel(uint32_t n, 
 //   A12 := L11^-1 (A12 - L[p, p-1] U[p-1, .]).
 // 4 warps; the updated operand goes through shared memory between the two products, and to the
 // backup.  The first product reads only what older panels left, so it runs before grid_wait, beside
-// the end of top_factor_kernel.  R = 16 at every size: the shortest chain per CTA, and the few SMs that the bulk update
-// leaves are shared most evenly (n = 2048: 957 us; 32 rows above 1024 rows 982, 64 above 1600 1008;
-// n = 4096: 3108, 3187, 3278).
+// the end of top_factor_kernel.  R = 16 at every size: the shortest chain per CTA, and the few SMs that
+// the bulk update leaves are shared most evenly (16, 32, 64 rows: n = 451 204, 214, 252 us; 2048 832, 897,
+// 1072; 4096 2921, 3084, 3518; 8192 16572, 16703, 17688).
 constexpr int kApplyRows = 16;
 constexpr int kApplyThreads = 128;
 constexpr size_t kApplySmem = (size_t)3 * NB * kPad * sizeof(double);
